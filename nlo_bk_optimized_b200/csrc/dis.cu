@@ -215,20 +215,28 @@ __global__ void table_initialize_kernel(double* table, int nr, int ny, double Y)
 // ===========================================================================
 // Pointwise integrands (the reference's dis_*_integrand operators)
 
+constexpr int kPointsThreads = 128;
+
 template <typename T, int TERM>
-__global__ void points_kernel(const DisArgs<T> args, InnerRule rule, const double* __restrict__ x, int64_t n,
+__global__ void __launch_bounds__(kPointsThreads, (warp_term<T, TERM>() ? 8 : 1)) points_kernel(const DisArgs<T> args, InnerRule rule, const double* __restrict__ x, int64_t n,
                               double* __restrict__ out)
 {
     constexpr int D = term_dims(TERM);
     __shared__ __align__(16) unsigned char raw[sizeof(DisArgs<T>)];
     DisArgs<T>& a = *reinterpret_cast<DisArgs<T>*>(raw);
+    __shared__ WarpShared<T, TERM, kPointsThreads> ws;
     if (threadIdx.x == 0) a = args;
+    ws.stage(rule);
     __syncthreads();
-    for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
+    // whole warps stay in the loop: a nested FP32 term is evaluated by its warp
+    for (int64_t base = blockIdx.x * (int64_t)blockDim.x; base < n; base += (int64_t)gridDim.x * blockDim.x) {
+        const int64_t i = base + threadIdx.x;
+        const bool on = i < n;
         double xl[D];
 #pragma unroll
-        for (int d = 0; d < D; ++d) xl[d] = x[i * D + d];
-        out[i] = (double)term_value<T, TERM>(a, xl, rule);
+        for (int d = 0; d < D; ++d) xl[d] = on ? x[i * D + d] : 0.5;
+        const double v = (double)term_value_warp<T, TERM>(a, on, xl, rule, ws);
+        if (on) out[i] = v;
     }
 }
 
@@ -297,7 +305,7 @@ __global__ void gauss_legendre_kernel(const DisArgs<T>* __restrict__ args, Inner
 template <typename T, int TERM>
 constexpr int vegas_min_blocks()
 {
-    return sizeof(T) == 4 && TERM <= kTermDip2 ? 4 : 3;
+    return sizeof(T) == 4 && (TERM <= kTermDip2 || warp_term<T, TERM>()) ? 4 : 3;
 }
 
 template <typename T, int TERM>
@@ -329,7 +337,9 @@ __global__ void __launch_bounds__(kVegasThreads, (vegas_min_blocks<T, TERM>())) 
     if (threadIdx.x < D) ssh[threadIdx.x] = sd.shift[threadIdx.x];
     __shared__ __align__(16) unsigned char raw[sizeof(DisArgs<T>)];
     DisArgs<T>& a = *reinterpret_cast<DisArgs<T>*>(raw);
+    __shared__ WarpShared<T, TERM, kVegasThreads> ws;
     if (threadIdx.x == 0) a = args[job];
+    ws.stage(rule);
     __syncthreads();
 
     const uint64_t chunk = (samples + blocks_per_job - 1) / blocks_per_job;
@@ -360,8 +370,7 @@ __global__ void __launch_bounds__(kVegasThreads, (vegas_min_blocks<T, TERM>())) 
                 bin[d] = b;
             }
         }
-        double w = 0.0;
-        if (active) w = (double)term_value<T, TERM>(a, xl, rule) * inv_density;
+        const double w = (double)term_value_warp<T, TERM>(a, active, xl, rule, ws) * inv_density;
         tot += w;
         tot2 += w * w;
         // deterministic warp histogram: lanes that share a bin add in lane order
@@ -502,10 +511,9 @@ template <typename T, int TERM>
 cudaError_t launch_points_t(const void* args, const InnerRule& rule, const double* x, int64_t n, double* out,
                             cudaStream_t stream)
 {
-    const int threads = 128;
-    int64_t blocks = (n + threads - 1) / threads;
+    int64_t blocks = (n + kPointsThreads - 1) / kPointsThreads;
     blocks = blocks > 4096 ? 4096 : (blocks < 1 ? 1 : blocks);
-    points_kernel<T, TERM><<<(unsigned)blocks, threads, 0, stream>>>(*static_cast<const DisArgs<T>*>(args), rule, x, n,
+    points_kernel<T, TERM><<<(unsigned)blocks, kPointsThreads, 0, stream>>>(*static_cast<const DisArgs<T>*>(args), rule, x, n,
                                                                      out);
     return cudaGetLastError();
 }

@@ -8,7 +8,7 @@
 //   (Abramowitz & Stegun 9.6.10-9.6.11) and exp(-x) x^{-1/2} g_nu(2/x) above, with g_nu
 //   a Chebyshev interpolant (FP64, Clenshaw) or a least-squares polynomial (FP32) fitted
 //   by gen_special_tables.py against 50-digit values; relative error <= 1.3e-15 (FP64)
-//   and <= 8e-7 (FP32) on (0, 500].
+//   and <= 8e-7 (FP32) on (0, 500].  bessel_k0_f1 is the FP32 form of the moment loop.
 // * Li2 by the Bernoulli series in u = -ln(1-x) ('t Hooft & Veltman 1979) after the
 //   inversion (x < -1) and reflection (x > 1/2) identities.
 #pragma once
@@ -183,6 +183,45 @@ __device__ __forceinline__ K01<float> bessel_k01_from_rcp(float x, float rx)
 }
 
 __device__ __forceinline__ K01<float> bessel_k01(float x) { return bessel_k01_from_rcp(x, rcp_approx_f(x)); }
+
+// K0(x) and F1(x) = x K1(x) of the moment loop, which takes them some 150 times a sample: rows
+// of cubics for e^x K0 and e^x F1 in shared memory, found by the top bits of x.  Against the
+// two-branch form above this needs a third of the instructions and no branch (lanes on both
+// sides of x = 2 ran both); it pays there because the lanes' arguments are neighbours, so
+// their rows lie in few bank groups.  Relative error <= 5e-7 on (0, 80].  The terms that
+// take the functions a few times a sample keep the other form.
+struct BesselRows {
+    float4 k0[nlo_special::kBesselRows], f1[nlo_special::kBesselRows];
+};
+
+__device__ __forceinline__ void stage_bessel_rows(BesselRows& t)
+{
+    using namespace nlo_special;
+    for (int i = threadIdx.x; i < kBesselRows; i += blockDim.x) {
+        t.k0[i] = reinterpret_cast<const float4*>(kBesselRowsK0F)[i];
+        t.f1[i] = reinterpret_cast<const float4*>(kBesselRowsF1F)[i];
+    }
+}
+
+__device__ __forceinline__ void bessel_k0_f1(const BesselRows& t, float x, float& k0, float& f1)
+{
+    using namespace nlo_special;
+    const unsigned bits = __float_as_uint(x);
+    // an x below the rows wraps to the last row and is replaced; one above them (K < e^-128)
+    // underflows in exp_neg_f whatever its row gives
+    const unsigned i = min((bits >> 19) - kBesselFirst, (unsigned)kBesselRows - 1u);
+    const float dx = x - __uint_as_float(bits & 0xfff80000u);
+    const float4 a = t.k0[i], b = t.f1[i];
+    const float e = exp_neg_f(x);
+    k0 = e * fmaf(dx, fmaf(dx, fmaf(dx, a.w, a.z), a.y), a.x);
+    f1 = e * fmaf(dx, fmaf(dx, fmaf(dx, b.w, b.z), b.y), b.x);
+    if (x < kBesselLow) {
+        const float x2 = x * x;
+        const float lg = lg2_approx_f(x) - 1.0f;
+        k0 = fmaf(-lg, horner(kI0SmallF, x2), horner(kQ0SmallF, x2));
+        f1 = fmaf(x2, fmaf(lg, horner(kI1SmallF, x2), horner(kQ1SmallF, x2)), 1.0f);
+    }
+}
 
 template <typename T>
 __device__ __forceinline__ T bessel_k0(T x)

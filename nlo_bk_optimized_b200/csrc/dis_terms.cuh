@@ -12,6 +12,8 @@
 // does not lose the small differences near the end points.
 #pragma once
 
+#include <type_traits>
+
 #include "dis_math.cuh"
 #include "dis_table.cuh"
 
@@ -65,6 +67,7 @@ struct DisArgs {
     // dipole
     bool table;
     GBWParams<T> gbw;
+    GBWParams<double> gbw64;
     double gbw_min_r, gbw_max_r;
     TableView tab;
 };
@@ -76,20 +79,25 @@ __device__ __forceinline__ T amplitude(const DisArgs<T>& a, double r, double Y)
     return gbw_amplitude(a.gbw, (T)r, (T)Y);
 }
 
-// The three dipoles of a qg sample at one rapidity: a table looks its rows up once.
-template <typename T>
-__device__ __forceinline__ void amplitudes3(const DisArgs<T>& a, double r01, double r02, double r21, double Y, T& N01,
-                                            T& N02, T& N21)
+// The three dipoles of a qg sample at one rapidity, in the arithmetic type A: a table looks its
+// rows up once.
+template <typename A, typename T>
+__device__ __forceinline__ void amplitudes3(const DisArgs<T>& a, double r01, double r02, double r21, double Y, A& N01,
+                                            A& N02, A& N21)
 {
     if (a.table) {
         const TableRow row = table_row(a.tab, Y);
-        N01 = (T)table_amplitude_at(a.tab, row, r01);
-        N02 = (T)table_amplitude_at(a.tab, row, r02);
-        N21 = (T)table_amplitude_at(a.tab, row, r21);
+        N01 = (A)table_amplitude_at(a.tab, row, r01);
+        N02 = (A)table_amplitude_at(a.tab, row, r02);
+        N21 = (A)table_amplitude_at(a.tab, row, r21);
+    } else if constexpr (sizeof(A) == 8) {
+        N01 = gbw_amplitude(a.gbw64, r01, Y);
+        N02 = gbw_amplitude(a.gbw64, r02, Y);
+        N21 = gbw_amplitude(a.gbw64, r21, Y);
     } else {
-        N01 = gbw_amplitude(a.gbw, (T)r01, (T)Y);
-        N02 = gbw_amplitude(a.gbw, (T)r02, (T)Y);
-        N21 = gbw_amplitude(a.gbw, (T)r21, (T)Y);
+        N01 = gbw_amplitude(a.gbw, (A)r01, (A)Y);
+        N02 = gbw_amplitude(a.gbw, (A)r02, (A)Y);
+        N21 = gbw_amplitude(a.gbw, (A)r21, (A)Y);
     }
 }
 
@@ -754,96 +762,217 @@ __device__ T l_i3(const Trip<T>& t, const GSet<T>& G1, const GSet<T>& G2)
                      - (T)2 * c * a * G1.g11[0] * G2.g11[1]));
 }
 
-// FP32 form of the moment loop.  Per node y the reciprocal 1/y is shared by the two sides;
-// per side the quantities that do not depend on y (M2 = Qbar^2 + m^2, its square root,
-// lambda m^2, x3^2, omega x2^2) are formed once.  With q = sqrt(B/y):
-//   z0 = sqrt(M2) q,  z1 = sqrt(A1) q,  z1 - z0 = q delta/(sqrt(A1)+sqrt(M2)),
-// so each (node, side) needs two square roots and two reciprocals besides the Bessel pairs.
-__device__ __forceinline__ K01<float> bessel_k01_rcp(float x, float& rx)
+// ---------------------------------------------------------------------------
+// FP32 moments, one warp per 32 samples: the lanes take the nodes of the inner rule, one side of
+// one sample ("segment") per half-warp.
+//
+// With a sample per lane every branch of an item (one node, one side) ran for the whole warp.
+// Along the nodes of one segment the branches are monotone in y, so 16 lanes take 16
+// neighbouring nodes, from the largest y down, and a segment ends at the first chunk whose
+// nodes are all negligible; the 64 segments of a warp are taken in the order of the branch
+// their last node needs, so that the two halves of the warp mostly agree.
+//
+// The moments, with s = z0^2 = M2 B/y, B = y x3^2 + omega x2^2 and z1^2 = s (1 + eps),
+// eps = y lambda m^2/M2, sqrt(y) cancelled and the constants 8 omega, 4 omega, 4, 2 last:
+//   G11 = 2 sum w/y K0(z1)             G21 = 4 sum w/B F1(z1)
+//   G12 = 4 omega sum w/(y B) D12      G22 = 8 omega sum w/B E22
+// F1(z) = z K1(z), D12 = F1(z1) - F1(z0), E22 = (A1 F(z1) - M2 F(z0))/y, F = K0 + 2 K1/z.
+// For small eps the differences cancel; the multiplication theorem (Abramowitz & Stegun 9.6.51)
+// gives them, and K0(z1), from K0 and K1 at z0 alone: with g = eps/2, M_k = z0^k K_k(z0)
+// (M_{k+1} = s M_{k-1} + 2 k M_k, no division) and Q_k = s M_k,
+//   K0(z1) = sum_k (-g)^k/k! M_k             D12 = sum_{k>0} (-g)^k/k! Q_{k-1}
+//   E22 = M2/y [-g M1 + sum_{k>1} (-g)^k/k! Q_{k-2}]
+// Taken through k = 7 where eps <= 0.2 and g z0 <= 0.45 (truncation below 2e-7; it covers
+// every node whose direct difference would lose more than a digit), and through k = 5 where
+// a whole chunk has eps <= 0.08 and g z0 <= 0.12.  A node is negligible where z0 exceeds its
+// smallest value over the segment (the last node's) by 32: its terms are below 1e-13 of it.
+// E22's direct form is A1 F(z1) - M2 F(z0) with F = K0 + 2 F1/z^2.
+// What bounds it: instruction issue.
+constexpr int kNodeLanes = 16;
+
+constexpr float kSeriesG = 0.1f, kSeriesGz = 0.45f;    // eps/2 and g z0 of the series
+constexpr float kShortG = 0.04f, kShortGz = 0.12f;     // ... through k = 5
+
+struct WarpSample {
+    // per side: M2, sqrt(M2), the z0 beyond which a node is negligible, lambda m^2/(2 M2);
+    // x3^2, omega x2^2, lambda m^2, -.  The first row holds the side's 4 sums after its segment.
+    float4 side[2][2];
+};
+
+// A warp's segments (2 sample + side) in the order they are taken.
+struct WarpOrder {
+    uint8_t segment[64];
+};
+
+// What the warps of a CTA share: the nodes as (y, 1/y, w, w/y) and the Bessel rows.
+struct MomentTables {
+    float4 nodes[kMaxInner];
+    BesselRows rows;
+};
+
+// Call once per CTA, before a barrier.
+__device__ __forceinline__ void stage_moment_tables(const InnerRule& rule, MomentTables& mt)
 {
-    rx = rcp_approx_f(x);
-    return bessel_k01_from_rcp(x, rx);
+    for (int i = threadIdx.x; i < rule.n; i += blockDim.x) {
+        const float y = (float)rule.y[i], w = (float)rule.w[i];
+        const float iy = rcp_approx_f(y);
+        mt.nodes[i] = make_float4(y, iy, w, w * iy);
+    }
+    stage_bessel_rows(mt.rows);
 }
 
-__device__ __forceinline__ GSet<float> g_moments_f32(const Trip<float>& t, const InnerRule& rule)
+// The sums a22, a12, a21, a11 of one segment over this lane's nodes.  SHORT: every node of both
+// halves' segments takes the series through k = 5.
+template <bool SHORT>
+__device__ __forceinline__ float4 segment_sums(const MomentTables& mt, int n, int l, float4 p, float4 r)
 {
-    // The side constants of the moments (8 omega, 4 omega, 4, 2) are applied after the
-    // loop, and sqrt(y) cancels between sqrt(A/B) = z sqrt(y)/B and the 1/sqrt(y) of the
-    // G functions:
-    //   G11 = 2 sum w/y K0(z1)             G21 = 4 sum w/B z1 K1(z1)
-    //   G12 = 4 omega sum w/(y B) D12      G22 = 8 omega sum w/B E
-    // with D12 = z1 K1(z1) - z0 K1(z0) (or the Euler-Maclaurin d1) and
-    // E = (A1 F(z1) - M2 F(z0))/y, F(z) = K0 + 2 K1/z (or d2/B).
-    float acc22[2], acc12[2], acc21[2], acc11[2];
-    float M2[2], sM2[2], lm2[2], x3[2], wx2[2];
-#pragma unroll
-    for (int s = 0; s < 2; ++s) {
-        acc22[s] = acc12[s] = acc21[s] = acc11[s] = 0.0f;
-        M2[s] = t.Qb2[s] + t.m2;
-        sM2[s] = sqrtf(M2[s]);
-        lm2[s] = t.lam[s] * t.m2;
-        x3[s] = t.x3sq[s];
-        wx2[s] = t.omega[s] * t.x2sq[s];
-    }
-    for (int i = 0; i < rule.n; ++i) {
-        const float y = (float)rule.y[i];
-        const float w = (float)rule.w[i];
-        const float iy = rcp_approx_f(y);
-        const float wiy = w * iy;
-#pragma unroll
-        for (int s = 0; s < 2; ++s) {
-            const float B = fmaf(y, x3[s], wx2[s]);
-            const float iB = rcp_approx_f(B);
-            const float q = sqrtf(B * iy);
-            const float delta = y * lm2[s];
-            const float Al = delta + M2[s];
-            const float sAl = sqrtf(Al);
-            const float z1 = sAl * q, z0 = sM2[s] * q;
-            float r1, r0;
-            const K01<float> kl = bessel_k01_rcp(z1, r1);
-            const K01<float> k0 = bessel_k01_rcp(z0, r0);
-            const float h = q * delta * rcp_approx_f(sAl + sM2[s]);
-            const float z1k1 = z1 * kl.k1;
-            float d12, e22;
-            if (h < 0.3f && h < 0.1f * z0) {
-                // Euler-Maclaurin integral of dF/dz over [z0, z1] (see f_differences_em)
-                const float h2 = h * h;
-                const float e2 = h2 * (1.0f / 12.0f), e4 = h2 * h2 * (1.0f / 720.0f);
-                const float d1 = 0.5f * h * (-z0 * k0.k0 - z1 * kl.k0) -
-                                 e2 * ((z1k1 - kl.k0) - (z0 * k0.k1 - k0.k0)) +
-                                 e4 * ((z1k1 - 2.0f * kl.k0 - kl.k1 * r1) - (z0 * k0.k1 - 2.0f * k0.k0 - k0.k1 * r0));
-                const float d2 = 0.5f * h * (-z0 * z0 * k0.k1 - z1 * z1k1) -
-                                 e2 * ((z1 * z1 * kl.k0 - z1k1) - (z0 * z0 * k0.k0 - z0 * k0.k1)) +
-                                 e4 * (((3.0f + z1 * z1) * kl.k0 - 4.0f * z1k1) -
-                                       ((3.0f + z0 * z0) * k0.k0 - 4.0f * z0 * k0.k1));
-                d12 = d1;
-                e22 = iB * d2;
+    float4 acc = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    for (int top = n - 1 - l; top + l >= 0; top -= kNodeLanes) {
+        const float4 nd = mt.nodes[top > 0 ? top : 0];
+        const float biy = fmaf(nd.x, r.x, r.y) * nd.y;  // B/y
+        const float rq = rsqrtf(biy);
+        const float sb = biy * rq;
+        const float z0 = p.y * sb;
+        const bool live = top >= 0 && !(z0 > p.z);
+        if (!__any_sync(0xffffffffu, live)) break;
+        const float g = nd.x * p.w;
+        bool series = true, longer = false;
+        if (!SHORT) {
+            const float gz = g * z0;
+            series = g <= kSeriesG && gz <= kSeriesGz;
+            longer = __any_sync(0xffffffffu, live && series && (g > kShortG || gz > kShortGz));
+        }
+        if (live) {
+            const float rb = rq * rq;  // y/B
+            float M0, M1;              // K0(z0), F1(z0)
+            bessel_k0_f1(mt.rows, z0, M0, M1);
+            float k0l, f1l, d12, e22;
+            if (SHORT || series) {
+                const float sq = p.x * biy;  // z0^2
+                const float Q0 = sq * M0, Q1 = sq * M1;
+                const float M2k = fmaf(2.0f, M1, Q0);
+                const float M3 = fmaf(4.0f, M2k, Q1);
+                const float Q2 = sq * M2k, Q3 = sq * M3;
+                const float M4 = fmaf(6.0f, M3, Q2);
+                const float M5 = fmaf(8.0f, M4, Q3);
+                float t0 = M5, t1 = sq * M4, t2 = Q3;
+                if (!SHORT && longer) {
+                    const float M6 = fmaf(10.0f, M5, t1), Q5 = sq * M5;
+                    const float M7 = fmaf(12.0f, M6, Q5);
+                    const float g7 = g * (1.0f / 7.0f), g6 = g * (1.0f / 6.0f);
+                    t0 = fmaf(-g6, fmaf(-g7, M7, M6), t0);
+                    t2 = fmaf(-g6, fmaf(-g7, Q5, t1), t2);
+                    t1 = fmaf(-g6, fmaf(-g7, sq * M6, Q5), t1);
+                }
+                const float g5 = g * 0.2f, g4 = g * 0.25f, g3 = g * (1.0f / 3.0f), g2 = g * 0.5f;
+                k0l = fmaf(-g, fmaf(-g2, fmaf(-g3, fmaf(-g4, fmaf(-g5, t0, M4), M3), M2k), M1), M0);
+                d12 = -g * fmaf(-g2, fmaf(-g3, fmaf(-g4, fmaf(-g5, t1, Q3), Q2), Q1), Q0);
+                e22 = -g * fmaf(-g2, fmaf(-g3, fmaf(-g4, fmaf(-g5, t2, Q2), Q1), Q0), M1);
+                e22 *= p.x * nd.y;
+                f1l = M1 + d12;
             } else {
-                d12 = z1k1 - z0 * k0.k1;
-                e22 = iy * (Al * fmaf(2.0f * kl.k1, r1, kl.k0) - M2[s] * fmaf(2.0f * k0.k1, r0, k0.k0));
+                const float Al = fmaf(nd.x, r.z, p.x);
+                const float z1 = (Al * rsqrtf(Al)) * sb;
+                bessel_k0_f1(mt.rows, z1, k0l, f1l);
+                d12 = f1l - M1;
+                // A1 F(z1) - M2 F(z0), F = K0 + 2 F1/z^2 and A1/z1^2 = M2/z0^2 = y/B
+                e22 = nd.y * fmaf(2.0f * rb, d12, Al * k0l - p.x * M0);
             }
-            const float wiB = w * iB;
-            acc22[s] = fmaf(wiB, e22, acc22[s]);
-            acc12[s] = fmaf(wiy * iB, d12, acc12[s]);
-            acc21[s] = fmaf(wiB, z1k1, acc21[s]);
-            acc11[s] = fmaf(wiy, kl.k0, acc11[s]);
+            const float iB = nd.y * rb;
+            const float wiB = nd.z * iB;
+            acc.x = fmaf(wiB, e22, acc.x);
+            acc.y = fmaf(nd.w * iB, d12, acc.y);
+            acc.z = fmaf(wiB, f1l, acc.z);
+            acc.w = fmaf(nd.w, k0l, acc.w);
         }
     }
-    GSet<float> m;
+    return acc;
+}
+
+// Moments of the samples of a warp's lanes (those with `on` set); every lane of the warp
+// calls it.  `slots`: 32 WarpSample of this warp.
+__device__ __forceinline__ GSet<float> g_moments_warp(bool on, const Trip<float>& t, const MomentTables& mt, int n,
+                                                      WarpSample* slots, WarpOrder& order)
+{
+    const int lane = threadIdx.x & 31;
+    const int half = lane >> 4, l = lane & (kNodeLanes - 1);
+    // a segment's place by its last node: 0 the short series throughout, 1 the series throughout,
+    // 2 and 3 the direct form for the last nodes and for most
+    int kind[2] = {-1, -1};
+    if (on) {
+        const float4 last = mt.nodes[n - 1];
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-        m.g22[s] = 8.0f * t.omega[s] * acc22[s];
-        m.g12[s] = 4.0f * t.omega[s] * acc12[s];
-        m.g21[s] = 4.0f * acc21[s];
-        m.g11[s] = 2.0f * acc11[s];
+        for (int q = 0; q < 2; ++q) {
+            const float M2 = t.Qb2[q] + t.m2;
+            const float rs = rsqrtf(M2);
+            const float sM = M2 * rs;
+            const float lm2 = t.lam[q] * t.m2;
+            const float wx2 = t.omega[q] * t.x2sq[q];
+            const float zmin = sM * sqrtf(fmaf(wx2, last.y, t.x3sq[q]));
+            const float hl = 0.5f * lm2 * (rs * rs);
+            slots[lane].side[q][0] = make_float4(M2, sM, zmin + 32.0f, hl);
+            slots[lane].side[q][1] = make_float4(t.x3sq[q], wx2, lm2, 0.0f);
+            // g z0 grows with y like g does: sqrt(y) at least
+            const float g = hl * last.x, gz = g * zmin;
+            kind[q] = g <= kShortG && gz <= kShortGz                         ? 0
+                      : g <= kSeriesG && gz <= kSeriesGz                     ? 1
+                      : g <= 8.0f * kSeriesG && gz <= 8.0f * kSeriesGz       ? 2
+                                                                             : 3;
+        }
     }
+    int total = 0, shorts = 0;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const unsigned mask = __ballot_sync(0xffffffffu, kind[q] == c);
+            if (kind[q] == c) order.segment[total + __popc(mask & ((1u << lane) - 1u))] = (uint8_t)(2 * lane + q);
+            total += __popc(mask);
+        }
+        if (c == 0) shorts = total;
+    }
+    __syncwarp();
+    for (int i = 0; i < total; i += 2) {
+        const bool mine = i + half < total;
+        const int seg = order.segment[mine ? i + half : i];
+        float4* side = slots[seg >> 1].side[seg & 1];
+        float4 p = side[0];
+        const float4 r = side[1];
+        if (!mine) p.z = -1.0f;  // an odd count: the second half of the last pair is dead
+        const float4 a = i + 2 <= shorts ? segment_sums<true>(mt, n, l, p, r) : segment_sums<false>(mt, n, l, p, r);
+        // the four sums over the 16 lanes: two are exchanged with the lane 8 away, one with the
+        // lane 4 away, then lane 4 k holds sum k
+        const bool up8 = (lane & 8) != 0, up4 = (lane & 4) != 0;
+        float u0 = up8 ? a.z : a.x, u1 = up8 ? a.w : a.y;
+        u0 += __shfl_xor_sync(0xffffffffu, up8 ? a.x : a.z, 8);
+        u1 += __shfl_xor_sync(0xffffffffu, up8 ? a.y : a.w, 8);
+        float v = up4 ? u1 : u0;
+        v += __shfl_xor_sync(0xffffffffu, up4 ? u0 : u1, 4);
+        v += __shfl_xor_sync(0xffffffffu, v, 2);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        // every lane has read the segment before the shuffles: its row takes the sums
+        if (mine && (lane & 3) == 0) reinterpret_cast<float*>(side)[l >> 2] = v;
+    }
+    __syncwarp();
+    GSet<float> m;
+    if (on) {
+#pragma unroll
+        for (int q = 0; q < 2; ++q) {
+            const float4 a = slots[lane].side[q][0];  // a22, a12, a21, a11
+            m.g22[q] = 8.0f * t.omega[q] * a.x;
+            m.g12[q] = 4.0f * t.omega[q] * a.y;
+            m.g21[q] = 4.0f * a.z;
+            m.g11[q] = 2.0f * a.w;
+        }
+    }
+    __syncwarp();
     return m;
 }
 
+// The FP64 build's moments (one lane per sample).
 template <typename T>
 __device__ __forceinline__ GSet<T> g_moments(const Trip<T>& t, const InnerRule& rule)
 {
-    if constexpr (sizeof(T) == 4) return g_moments_f32(t, rule);
     GSet<T> m;
 #pragma unroll
     for (int s = 0; s < 2; ++s) m.g22[s] = m.g12[s] = m.g21[s] = m.g11[s] = (T)0;
@@ -862,103 +991,147 @@ __device__ __forceinline__ GSet<T> g_moments(const Trip<T>& t, const InnerRule& 
 }
 
 // integrand_qgunsub_massive (dis/observables.py:175-250) and the nested forms
-// (integrand_qg_nested_massive, :253-331)
+// (integrand_qg_nested_massive, :253-331): the physical point of a unit-cube point in FP64;
+// false where the integrand vanishes.
+struct QgGeometry {
+    double z1, z2, x01, x02, x21, Y, jac;
+};
+
+template <typename T>
+__device__ __forceinline__ bool qg_geometry(const DisArgs<T>& a, const double* x, QgGeometry& g)
+{
+    const double z2min = a.z2min;
+    if (z2min > 1.0) return false;
+    g.z1 = (1.0 - z2min) * x[0];
+    g.z2 = (1.0 - g.z1 - z2min) * x[1] + z2min;
+    g.x01 = a.maxr * x[2];
+    g.x02 = a.maxr * x[3];
+    const double phi = 2.0 * kPi * x[4];
+    const double x21sq = g.x01 * g.x01 + g.x02 * g.x02 - 2.0 * g.x01 * g.x02 * ::cos(phi);
+    g.x21 = ::sqrt(x21sq > 0.0 ? x21sq : 0.0);
+    g.jac = (1.0 - z2min) * (1.0 - g.z1 - z2min) * g.x01 * g.x02 * a.maxr * a.maxr * 2.0 * kPi;
+    g.Y = ::log(a.W2 * g.z2 / kQ0sqr);
+    return g.Y >= 0.0;
+}
+
+// Its amplitudes, coupling and tripole geometry.
+template <typename T>
+struct QgPoint {
+    Trip<T> t;
+    T x01sq, N01, N012, af;
+    double jac_z2;  // Jacobian / z2
+};
+
+// N01 and the tripole factor N012.
+template <typename A, typename T>
+__device__ __forceinline__ void qg_amplitudes(const DisArgs<T>& a, const QgGeometry& g, A& N01, A& N012)
+{
+    A N02, N21;
+    amplitudes3(a, g.x01, g.x02, g.x21, g.Y, N01, N02, N21);
+    const A S01 = (A)1 - N01, S02 = (A)1 - N02, S12 = (A)1 - N21;
+    N012 = a.finite_nc ? (A)1 - (A)(kNc / (2.0 * kCF)) * (S02 * S12 - S01 / (A)(kNc * kNc)) : (A)1 - S02 * S12;
+    N01 = (A)1 - S01;
+}
+
+// Everything but the amplitudes.
+template <typename T>
+__device__ __forceinline__ void qg_point(const DisArgs<T>& a, const QgGeometry& g, QgPoint<T>& p)
+{
+    const double ra = a.parent_coupling ? g.x01 : fmin(g.x01, fmin(g.x02, g.x21));
+    p.af = alpha_bar(a, (T)ra);
+    p.t = make_trip<T>(a.Q2, a.mf, g.z1, g.z2, g.x01 * g.x01, g.x02 * g.x02, g.x21 * g.x21);
+    p.x01sq = (T)(g.x01 * g.x01);
+    p.jac_z2 = g.jac / g.z2;
+}
+
+template <typename T>
+__device__ __forceinline__ T qg_i1(bool transverse, const Trip<T>& t, T x01sq, T N01, T N012)
+{
+    T uvsub, trip;
+    if (transverse)
+        t_i1(t, x01sq, uvsub, trip);
+    else
+        l_i1(t, x01sq, uvsub, trip);
+    return N01 * uvsub + N012 * trip;
+}
+
+template <typename T, int TERM>
+__device__ __forceinline__ T qg_nested_value(const DisArgs<T>& a, const QgPoint<T>& p, const GSet<T>& G)
+{
+    if constexpr (TERM == kTermI2N)
+        return p.N012 * (a.transverse ? t_i2(p.t, G) : l_i2(p.t, G));
+    else
+        return p.N012 * (a.transverse ? t_i3(p.t, G, G) : l_i3(p.t, G, G));
+}
+
+template <typename T>
+__device__ __forceinline__ T qg_scaled(const QgPoint<T>& p, T v)
+{
+    const T out = v * (T)p.jac_z2 * p.af;
+    return DM<T>::finite(out) ? out : (T)0;
+}
+
 template <typename T, int TERM>
 __device__ T qg_term(const DisArgs<T>& a, const double* x, const InnerRule& rule)
 {
-    const double z2min = a.z2min;
-    if (z2min > 1.0) return (T)0;
-    const double z1 = (1.0 - z2min) * x[0];
-    const double z2 = (1.0 - z1 - z2min) * x[1] + z2min;
-    const double x01 = a.maxr * x[2];
-    const double x02 = a.maxr * x[3];
-    const double phi = 2.0 * kPi * x[4];
-    const double x01sq = x01 * x01, x02sq = x02 * x02;
-    double x21sq = x01sq + x02sq - 2.0 * x01 * x02 * ::cos(phi);
-    x21sq = x21sq > 0.0 ? x21sq : 0.0;
-    const double x21 = ::sqrt(x21sq);
-    const double jac = (1.0 - z2min) * (1.0 - z1 - z2min) * x01 * x02 * a.maxr * a.maxr * 2.0 * kPi;
-    const double Y = ::log(a.W2 * z2 / kQ0sqr);
-    if (!(Y >= 0.0)) return (T)0;
-    T N01, N02, N21;
-    amplitudes3(a, x01, x02, x21, Y, N01, N02, N21);
-    const T S01 = (T)1 - N01;
-    const T S02 = (T)1 - N02;
-    const T S12 = (T)1 - N21;
-    const T N012 = a.finite_nc ? (T)1 - (T)(kNc / (2.0 * kCF)) * (S02 * S12 - S01 / (T)(kNc * kNc))
-                               : (T)1 - S02 * S12;
-    const double ra = a.parent_coupling ? x01 : fmin(x01, fmin(x02, x21));
-    const T af = alpha_bar(a, (T)ra);
-    const Trip<T> t = make_trip<T>(a.Q2, a.mf, z1, z2, x01sq, x02sq, x21sq);
+    QgGeometry g;
+    if (!qg_geometry(a, x, g)) return (T)0;
+    QgPoint<T> p;
+    qg_amplitudes(a, g, p.N01, p.N012);
+    qg_point(a, g, p);
     T v;
     if constexpr (TERM == kTermI1) {
-        T uvsub, trip;
-        if (a.transverse)
-            t_i1(t, (T)x01sq, uvsub, trip);
-        else
-            l_i1(t, (T)x01sq, uvsub, trip);
-        v = ((T)1 - S01) * uvsub + N012 * trip;
-    } else if constexpr (TERM == kTermI2 || TERM == kTermI2N) {
-        GSet<T> G;
-        if constexpr (TERM == kTermI2)
-            G = g_values(t, (T)x[5]);
-        else
-            G = g_moments(t, rule);
-        v = N012 * (a.transverse ? t_i2(t, G) : l_i2(t, G));
+        v = qg_i1(a.transverse, p.t, p.x01sq, p.N01, p.N012);
+    } else if constexpr (TERM == kTermI2) {
+        const GSet<T> G = g_values(p.t, (T)x[5]);
+        v = p.N012 * (a.transverse ? t_i2(p.t, G) : l_i2(p.t, G));
+    } else if constexpr (TERM == kTermI3) {
+        const GSet<T> G1 = g_values(p.t, (T)x[5]);
+        const GSet<T> G2 = g_values(p.t, (T)x[6]);
+        v = p.N012 * (a.transverse ? t_i3(p.t, G1, G2) : l_i3(p.t, G1, G2));
     } else {
-        if constexpr (TERM == kTermI3) {
-            const GSet<T> G1 = g_values(t, (T)x[5]);
-            const GSet<T> G2 = g_values(t, (T)x[6]);
-            v = N012 * (a.transverse ? t_i3(t, G1, G2) : l_i3(t, G1, G2));
-        } else {
-            const GSet<T> G = g_moments(t, rule);
-            v = N012 * (a.transverse ? t_i3(t, G, G) : l_i3(t, G, G));
-        }
+        v = qg_nested_value<T, TERM>(a, p, g_moments(p.t, rule));
     }
-    const T out = v * (T)(jac / z2) * af;
-    return DM<T>::finite(out) ? out : (T)0;
+    return qg_scaled(p, v);
 }
 
 // I1, and I2 and I3 with the inner rule, at one point: the map, the amplitudes, the
 // coupling and the tripole geometry are shared, and I2 and I3 use one moment set (the
-// combined evaluation of the fixed-Sobol path, dis/fixed_sobol.py:273-368).
-template <typename T>
-__device__ void qg_triple(const DisArgs<T>& a, const double* x, const InnerRule& rule, T out[3])
+// combined evaluation of the fixed-Sobol path, dis/fixed_sobol.py:273-368).  Every lane of
+// the warp calls it; `on` marks the lanes with a point.
+//
+// The FP32 build takes I1 and the amplitudes in FP64 (the FP64 "sensitive" part of the
+// reference's fused path): I1's parts cancel to 1/10 .. 1/100 of themselves, and 1 - S with
+// S = 1 - N leaves 1e-3 of N012 for dipoles of N ~ 1e-4; in FP32 the remainder was 1e-6 .. 6e-5 of
+// the total and, through the training scores, moved the grid.
+template <typename T, class Shared>
+__device__ void qg_triple(const DisArgs<T>& a, bool on, const double* x, const InnerRule& rule, Shared& ws, T out[3])
 {
     out[0] = out[1] = out[2] = (T)0;
-    const double z2min = a.z2min;
-    if (z2min > 1.0) return;
-    const double z1 = (1.0 - z2min) * x[0];
-    const double z2 = (1.0 - z1 - z2min) * x[1] + z2min;
-    const double x01 = a.maxr * x[2];
-    const double x02 = a.maxr * x[3];
-    const double phi = 2.0 * kPi * x[4];
-    const double x01sq = x01 * x01, x02sq = x02 * x02;
-    double x21sq = x01sq + x02sq - 2.0 * x01 * x02 * ::cos(phi);
-    x21sq = x21sq > 0.0 ? x21sq : 0.0;
-    const double x21 = ::sqrt(x21sq);
-    const double jac = (1.0 - z2min) * (1.0 - z1 - z2min) * x01 * x02 * a.maxr * a.maxr * 2.0 * kPi;
-    const double Y = ::log(a.W2 * z2 / kQ0sqr);
-    if (!(Y >= 0.0)) return;
-    T N01, N02, N21;
-    amplitudes3(a, x01, x02, x21, Y, N01, N02, N21);
-    const T S01 = (T)1 - N01;
-    const T S02 = (T)1 - N02;
-    const T S12 = (T)1 - N21;
-    const T N012 = a.finite_nc ? (T)1 - (T)(kNc / (2.0 * kCF)) * (S02 * S12 - S01 / (T)(kNc * kNc))
-                               : (T)1 - S02 * S12;
-    const double ra = a.parent_coupling ? x01 : fmin(x01, fmin(x02, x21));
-    const T scale = alpha_bar(a, (T)ra) * (T)(jac / z2);
-    const Trip<T> t = make_trip<T>(a.Q2, a.mf, z1, z2, x01sq, x02sq, x21sq);
-    T uvsub, trip;
-    if (a.transverse)
-        t_i1(t, (T)x01sq, uvsub, trip);
-    else
-        l_i1(t, (T)x01sq, uvsub, trip);
-    const GSet<T> G = g_moments(t, rule);
-    const T i1 = (((T)1 - S01) * uvsub + N012 * trip) * scale;
-    const T i2 = N012 * (a.transverse ? t_i2(t, G) : l_i2(t, G)) * scale;
-    const T i3 = N012 * (a.transverse ? t_i3(t, G, G) : l_i3(t, G, G)) * scale;
+    QgGeometry g;
+    on = on && qg_geometry(a, x, g);
+    QgPoint<T> p;
+    T i1 = (T)0;
+    if (on) {
+        double N01, N012;
+        qg_amplitudes(a, g, N01, N012);
+        qg_point(a, g, p);
+        p.N012 = (T)N012;
+        const double x01sq = g.x01 * g.x01;
+        const Trip<double> t = make_trip<double>(a.Q2, a.mf, g.z1, g.z2, x01sq, g.x02 * g.x02, g.x21 * g.x21);
+        i1 = (T)qg_i1(a.transverse, t, x01sq, N01, N012);
+    }
+    GSet<T> G;
+    if constexpr (sizeof(T) == 4) {
+        G = ws.moments(on, p.t, rule.n);
+    } else if (on) {
+        G = g_moments(p.t, rule);
+    }
+    if (!on) return;
+    const T scale = p.af * (T)p.jac_z2;
+    i1 *= scale;
+    const T i2 = qg_nested_value<T, kTermI2N>(a, p, G) * scale;
+    const T i3 = qg_nested_value<T, kTermI3N>(a, p, G) * scale;
     out[0] = DM<T>::finite(i1) ? i1 : (T)0;
     out[1] = DM<T>::finite(i2) ? i2 : (T)0;
     out[2] = DM<T>::finite(i3) ? i3 : (T)0;
@@ -977,6 +1150,51 @@ __device__ __forceinline__ T term_value(const DisArgs<T>& a, const double* x, co
         return dip_term<T, 2>(a, x);
     else
         return qg_term<T, TERM>(a, x, rule);
+}
+
+// The terms whose FP32 integrand is evaluated by whole warps (g_moments_warp).
+template <typename T, int TERM>
+constexpr bool warp_term()
+{
+    return sizeof(T) == 4 && (TERM == kTermI2N || TERM == kTermI3N);
+}
+
+// What a CTA of THREADS threads that evaluates TERM keeps in shared memory for it.
+struct NoShared {
+    __device__ __forceinline__ void stage(const InnerRule&) {}
+};
+template <int THREADS>
+struct MomentShared {
+    MomentTables mt;
+    WarpSample slots[THREADS];
+    WarpOrder order[THREADS / 32];
+    __device__ __forceinline__ void stage(const InnerRule& rule) { stage_moment_tables(rule, mt); }
+    __device__ __forceinline__ GSet<float> moments(bool on, const Trip<float>& t, int n)
+    {
+        return g_moments_warp(on, t, mt, n, slots + (threadIdx.x & ~31), order[threadIdx.x >> 5]);
+    }
+};
+template <typename T, int TERM, int THREADS>
+using WarpShared = std::conditional_t<warp_term<T, TERM>(), MomentShared<THREADS>, NoShared>;
+
+// term_value for the lanes of a warp with `on` set (0 for the others); every lane calls it.
+template <typename T, int TERM, class Shared>
+__device__ __forceinline__ T term_value_warp(const DisArgs<T>& a, bool on, const double* x, const InnerRule& rule,
+                                             Shared& ws)
+{
+    if constexpr (warp_term<T, TERM>()) {
+        QgGeometry g;
+        on = on && qg_geometry(a, x, g);
+        QgPoint<T> p;
+        if (on) {
+            qg_amplitudes(a, g, p.N01, p.N012);
+            qg_point(a, g, p);
+        }
+        const GSet<T> G = ws.moments(on, p.t, rule.n);
+        return on ? qg_scaled(p, qg_nested_value<T, TERM>(a, p, G)) : (T)0;
+    } else {
+        return on ? term_value<T, TERM>(a, x, rule) : (T)0;
+    }
 }
 
 }  // namespace dis

@@ -12,6 +12,11 @@ as the ground truth; nothing is taken from another library's tables.
   [0, 1] with g_nu(0) = sqrt(pi/2).  FP64: Chebyshev interpolant of g_nu in y = 2s - 1
   (Clenshaw recurrence on the device).  FP32: least-squares polynomial in s on Chebyshev
   nodes (Horner on the device).
+* A second FP32 form serves the moments of the inner rule, where the lanes of a warp hold
+  neighbouring arguments and a lookup costs little: exp(x) K0(x) and exp(x) x K1(x) as cubics
+  in x - x_i on the intervals of 1/16 octave that the top 13 bits of x name, from 2^-7 to 2^7
+  (least squares in relative error, below 4e-8); under 2^-7, polynomials in x^2 of the parts of
+  the ascending series (ln 2 folded in, since the device takes log2 x).
 * Li2 uses the Bernoulli-number series Li2(x) = sum_n B_n u^{n+1} / (n+1)!, u = -ln(1-x)
   ('t Hooft & Veltman, Nucl. Phys. B153 (1979) 365), after the standard reflection and
   inversion identities have brought x into [-1, 1/2].
@@ -41,6 +46,9 @@ SERIES_TERMS_F64 = 14
 SERIES_TERMS_F32 = 8
 CHEB_TERMS_F64 = 24
 POLY_DEGREE_F32 = 9
+SMALL_DEGREE_F32 = 1         # I0, Q0, I1, Q1 parts on x <= 2^-7
+ROWS_LOW, ROWS_HIGH = -7, 7  # octaves of the lookup
+ROWS_PER_OCTAVE = 16
 BERNOULLI_TERMS_F64 = 20
 BERNOULLI_TERMS_F32 = 9
 
@@ -121,6 +129,37 @@ def cheb_nodes(a, b, m: int):
     return [a + (b - a) * (mp.cos(mp.pi * (k + mp.mpf(1) / 2) / m) + 1) / 2 for k in range(m)]
 
 
+def small_tables():
+    """The parts of K0 = -(log2 x - 1) P0 + R0 and x K1 = 1 + x^2 ((log2 x - 1) P1 + R1) on
+    0 < x <= 2^ROWS_LOW as polynomials in x^2."""
+    ln2 = mp.log(2)
+    parts = (
+        lambda x: ln2 * mp.besseli(0, x),
+        lambda x: mp.besselk(0, x) + mp.log(x / 2) * mp.besseli(0, x),
+        lambda x: ln2 * mp.besseli(1, x) / x,
+        lambda x: (mp.besselk(1, x) - 1 / x - mp.log(x / 2) * mp.besseli(1, x)) / x,
+    )
+    ts = cheb_nodes(mp.mpf(0), mp.mpf(4) ** ROWS_LOW, 8 * (SMALL_DEGREE_F32 + 1))
+    return [least_squares(ts, [part(mp.sqrt(t)) for t in ts], lambda t, j: t**j, [1] * len(ts), SMALL_DEGREE_F32)
+            for part in parts]
+
+
+def row_tables():
+    """Cubic coefficients in x - x_i of exp(x) K0(x) and exp(x) x K1(x), row after row."""
+    tables = ([], [])
+    with mp.workdps(20):
+        ts = cheb_nodes(mp.mpf(0), mp.mpf(1), 6)
+        for octave in range(ROWS_LOW, ROWS_HIGH):
+            for k in range(ROWS_PER_OCTAVE):
+                step = mp.mpf(2) ** octave / ROWS_PER_OCTAVE
+                x0 = mp.mpf(2) ** octave + k * step
+                for nu, table in enumerate(tables):
+                    fs = [mp.exp(x) * mp.besselk(nu, x) * x**nu for x in (x0 + t * step for t in ts)]
+                    c = least_squares(ts, fs, lambda t, j: t**j, [1 / f for f in fs], 3)
+                    table += [v / step**j for j, v in enumerate(c)]
+    return tables
+
+
 def dla_tables():
     v0 = mp.mpf(DLA_T0) ** 2 / 4
     vs = cheb_nodes(-v0, v0, 8 * (DLA_POLY_DEGREE + 1))
@@ -178,12 +217,23 @@ def main() -> None:
     for name, table in (("kI0Series", i0), ("kQ0Series", q0), ("kI1Series", i1), ("kQ1Series", q1)):
         short = table[:SERIES_TERMS_F32]
         out += [f"__device__ constexpr float {name}F[{SERIES_TERMS_F32}] = {{", fmt(short, "f"), "};"]
+    for name, table in zip(("kI0SmallF", "kQ0SmallF", "kI1SmallF", "kQ1SmallF"), small_tables()):
+        out += [f"__device__ constexpr float {name}[{len(table)}] = {{", fmt(table, "f"), "};"]
     for nu in (0, 1):
         out += [f"__device__ constexpr double kK{nu}Cheb[{CHEB_TERMS_F64}] = {{",
                 fmt(chebyshev(nu, CHEB_TERMS_F64)), "};"]
     for nu in (0, 1):
         out += [f"__device__ constexpr float kK{nu}PolyF[{POLY_DEGREE_F32 + 1}] = {{",
                 fmt(poly_fit(nu, POLY_DEGREE_F32), "f"), "};"]
+    rows = (ROWS_HIGH - ROWS_LOW) * ROWS_PER_OCTAVE
+    out += ["", f"constexpr int kBesselRows = {rows};",
+            f"constexpr unsigned kBesselFirst = {(127 + ROWS_LOW) * ROWS_PER_OCTAVE}u;  // the top 13 bits of 2^{ROWS_LOW}",
+            f"constexpr float kBesselLow = {float(mp.mpf(2) ** ROWS_LOW)!r}f;"]
+    for name, table in zip(("kBesselRowsK0F", "kBesselRowsF1F"), row_tables()):
+        items = [mp.nstr(v, 10, min_fixed=-1, max_fixed=-1) + "f" for v in table]
+        out += [f"__device__ const __align__(16) float {name}[{len(table)}] = {{"]
+        out += ["    " + ", ".join(items[i : i + 8]) + "," for i in range(0, len(items), 8)]
+        out += ["};"]
     out += [f"__device__ constexpr double kLi2Bernoulli[{BERNOULLI_TERMS_F64}] = {{",
             fmt(bernoulli_tables(BERNOULLI_TERMS_F64)), "};"]
     out += [f"__device__ constexpr float kLi2BernoulliF[{BERNOULLI_TERMS_F32}] = {{",
