@@ -1071,28 +1071,61 @@ __device__ __forceinline__ T qg_scaled(const QgPoint<T>& p, T v)
     return DM<T>::finite(out) ? out : (T)0;
 }
 
+// One lane per sample (the FP64 nested forms among it).
 template <typename T, int TERM>
 __device__ T qg_term(const DisArgs<T>& a, const double* x, const InnerRule& rule)
 {
-    QgGeometry g;
-    if (!qg_geometry(a, x, g)) return (T)0;
-    QgPoint<T> p;
-    qg_amplitudes(a, g, p.N01, p.N012);
-    qg_point(a, g, p);
+    const double z2min = a.z2min;
+    if (z2min > 1.0) return (T)0;
+    const double z1 = (1.0 - z2min) * x[0];
+    const double z2 = (1.0 - z1 - z2min) * x[1] + z2min;
+    const double x01 = a.maxr * x[2];
+    const double x02 = a.maxr * x[3];
+    const double phi = 2.0 * kPi * x[4];
+    const double x01sq = x01 * x01, x02sq = x02 * x02;
+    double x21sq = x01sq + x02sq - 2.0 * x01 * x02 * ::cos(phi);
+    x21sq = x21sq > 0.0 ? x21sq : 0.0;
+    const double x21 = ::sqrt(x21sq);
+    const double jac = (1.0 - z2min) * (1.0 - z1 - z2min) * x01 * x02 * a.maxr * a.maxr * 2.0 * kPi;
+    const double Y = ::log(a.W2 * z2 / kQ0sqr);
+    if (!(Y >= 0.0)) return (T)0;
+    T N01, N02, N21;
+    amplitudes3(a, x01, x02, x21, Y, N01, N02, N21);
+    const T S01 = (T)1 - N01;
+    const T S02 = (T)1 - N02;
+    const T S12 = (T)1 - N21;
+    const T N012 = a.finite_nc ? (T)1 - (T)(kNc / (2.0 * kCF)) * (S02 * S12 - S01 / (T)(kNc * kNc))
+                               : (T)1 - S02 * S12;
+    const double ra = a.parent_coupling ? x01 : fmin(x01, fmin(x02, x21));
+    const T af = alpha_bar(a, (T)ra);
+    const Trip<T> t = make_trip<T>(a.Q2, a.mf, z1, z2, x01sq, x02sq, x21sq);
     T v;
     if constexpr (TERM == kTermI1) {
-        v = qg_i1(a.transverse, p.t, p.x01sq, p.N01, p.N012);
-    } else if constexpr (TERM == kTermI2) {
-        const GSet<T> G = g_values(p.t, (T)x[5]);
-        v = p.N012 * (a.transverse ? t_i2(p.t, G) : l_i2(p.t, G));
-    } else if constexpr (TERM == kTermI3) {
-        const GSet<T> G1 = g_values(p.t, (T)x[5]);
-        const GSet<T> G2 = g_values(p.t, (T)x[6]);
-        v = p.N012 * (a.transverse ? t_i3(p.t, G1, G2) : l_i3(p.t, G1, G2));
+        T uvsub, trip;
+        if (a.transverse)
+            t_i1(t, (T)x01sq, uvsub, trip);
+        else
+            l_i1(t, (T)x01sq, uvsub, trip);
+        v = ((T)1 - S01) * uvsub + N012 * trip;
+    } else if constexpr (TERM == kTermI2 || TERM == kTermI2N) {
+        GSet<T> G;
+        if constexpr (TERM == kTermI2)
+            G = g_values(t, (T)x[5]);
+        else
+            G = g_moments(t, rule);
+        v = N012 * (a.transverse ? t_i2(t, G) : l_i2(t, G));
     } else {
-        v = qg_nested_value<T, TERM>(a, p, g_moments(p.t, rule));
+        if constexpr (TERM == kTermI3) {
+            const GSet<T> G1 = g_values(t, (T)x[5]);
+            const GSet<T> G2 = g_values(t, (T)x[6]);
+            v = N012 * (a.transverse ? t_i3(t, G1, G2) : l_i3(t, G1, G2));
+        } else {
+            const GSet<T> G = g_moments(t, rule);
+            v = N012 * (a.transverse ? t_i3(t, G, G) : l_i3(t, G, G));
+        }
     }
-    return qg_scaled(p, v);
+    const T out = v * (T)(jac / z2) * af;
+    return DM<T>::finite(out) ? out : (T)0;
 }
 
 // I1, and I2 and I3 with the inner rule, at one point: the map, the amplitudes, the

@@ -37,4 +37,5 @@ def test_moments_vs_oracle(inner, count, mass):
             got = integrand_qg_nested_massive(points, Q2, xbj, pol, quark, term, GBW(Qs0sqr=0.25, lambda_=0.29),
                                               config).double().cpu().numpy()
             ref = od.qg_integrand(x, kin, term + "n", od.GBWDipole(qs0sqr=0.25, lam=0.29), points=inner)
-            assert np.linalg.norm(got - ref) <= 1e-5 * np.linalg.norm(ref), (pol, term)
+            floor = np.sqrt(count) * np.finfo(np.float32).tiny  # the device flushes what FP32 cannot hold
+            assert np.linalg.norm(got - ref) <= 1e-5 * np.linalg.norm(ref) + floor, (pol, term)
