@@ -723,7 +723,7 @@ size_t nlo_bk_vegas_workspace_bytes(int32_t points, const nlo_bk_vegas_options* 
 {
     std::string why;
     if (points < 3 || !check_vegas(options, why)) return 0;
-    return nlo_bk_rhs_workspace_bytes(points) + align_up(bk_vegas_scratch_bytes(points, options->bins));
+    return nlo_bk_rhs_workspace_bytes(points) + align_up(bk_vegas_scratch_bytes(points, *options));
 }
 
 // The Vegas buffers at the end of the workspace (after the right-hand side and stage rows);

@@ -148,16 +148,14 @@ struct BkVegasCall {
     double* state = nullptr;   // [points][stride], persistent grids
     int stride = 0;
     int blocks_per_job = 1;
-    double* partial = nullptr;  // [points][blocks][4 + 4 bins]
-    double* reduced = nullptr;  // [points][4 + 4 bins]
-    int32_t* counts = nullptr;  // [points][4 bins]
-    double* replica_state = nullptr;  // [points][stride], the replicas' fresh grids
+    double* partial = nullptr;  // [integrals][blocks][4 + 4 bins]
+    int32_t* counts = nullptr;  // [integrals][4 bins]
+    double* replica_state = nullptr;  // [replicas run together][points][stride], their fresh grids
     double* replica_acc = nullptr;    // [points][3], the replica refinement's sums
     const SobolDirsArg* replica_dirs = nullptr;  // [options.replicas]
 };
 size_t bk_vegas_state_doubles(int bins);
-int bk_vegas_blocks_per_job(int points);
-size_t bk_vegas_scratch_bytes(int points, int bins);
+size_t bk_vegas_scratch_bytes(int points, const nlo_bk_vegas_options& options);
 BkVegasCall bk_vegas_carve(void* scratch, int points, const nlo_bk_vegas_options& options, double* state);
 // Vegas K2+Kf of the active parents i % shards == shard of N into out[points][3] = [value, 0,
 // error^2] (zeros elsewhere).

@@ -7,13 +7,13 @@
 // per-parent vegas_states of bk/evolution.py:85-100 and 354-424).
 //
 // Every active parent is one integral with its own grid; all of them run in the same
-// launches.  A round (the warm-up, or one iteration) is three launches: the round kernel
-// (grid: CTAs per parent x grid points) maps scrambled Sobol points through the parent's
+// launches.  A round (the warm-up, or one iteration) is two launches: the round kernel
+// (grid: CTAs per parent x integrals) maps scrambled Sobol points through the parent's
 // grid, evaluates the full integrand and leaves per-CTA sums of w, w^2, w_K2, w_Kf and the
-// |w| histograms; a fixed-order reduction over the CTAs; and a finalize CTA per parent that
-// re-bins the grid and folds the iteration into the inverse-variance combination
-// (vegas_common.cuh, the code the DIS terms use).  Converged parents skip the remaining
-// rounds, so the host enqueues every round without synchronising.
+// |w| histograms; a finalize CTA per integral adds them in a fixed order, re-bins the grid
+// and folds the iteration into the inverse-variance combination (vegas_common.cuh, the code
+// the DIS terms use).  Converged parents skip the remaining rounds, so the host enqueues
+// every round without synchronising.
 //
 // Samples: the Sobol points of `dirs`, indices 0, 1, ... across the rounds of one
 // right-hand side (the warm-up first); every parent and every right-hand side starts again
@@ -21,11 +21,14 @@
 // call.  A coordinate u gives the bin floor(u bins) and the fraction u bins - bin.
 #include <cuda_runtime.h>
 
+#include <cstring>
+
 #include "common.cuh"
 #include "internal.h"
 #include "k2kf_integrand.cuh"
 #include "sobol.cuh"
 #include "vegas_common.cuh"
+#include "vegas_sampling.cuh"
 
 namespace nlo {
 
@@ -56,17 +59,19 @@ __device__ __forceinline__ bool parent_active(const double* N, int i, int shard,
     return i > 0 && N[i] <= 0.99999 && i % shards == shard;
 }
 
-// Per parent: mark whether it is integrated, reset the per-call sums, and either start a
-// uniform grid with the full warm-up or keep the stored grid with the reuse warm-up.
-// select (replica rounds): the parents to integrate are those with select[i * kRepStride] != 0.
+// Per integral: mark whether it is taken, reset the per-call sums, and either start a uniform
+// grid with the full warm-up or keep the stored grid with the reuse warm-up.  Integral
+// blockIdx.x is parent blockIdx.x % points.  select (replica rounds): the parents to integrate
+// are those with select[parent * kRepStride] != 0.
 __global__ void begin_kernel(const double* __restrict__ N, int points, int shard, int shards, double* state,
                              int stride, int bins, int reuse, uint64_t warmup, uint64_t reuse_warmup,
                              int32_t* __restrict__ counts, const double* __restrict__ select)
 {
     const int i = blockIdx.x;
+    const int parent = i % points;
     double* st = state + (size_t)i * stride;
     double* sc = st + kDims * (bins + 1);
-    const bool on = select ? select[(size_t)i * kRepStride] != 0.0 : parent_active(N, i, shard, shards);
+    const bool on = select ? select[(size_t)parent * kRepStride] != 0.0 : parent_active(N, parent, shard, shards);
     __syncthreads();
     const bool fresh = !reuse || sc[kBkHasGrid] == 0.0;
     if (on) {
@@ -90,6 +95,14 @@ __global__ void begin_kernel(const double* __restrict__ N, int points, int shard
     }
 }
 
+// Direction numbers of the integrals of one launch: set 0 of the main integrals, set g of the
+// g-th replica (integral / points).
+template <int SETS>
+struct BkDirs {
+    uint32_t state[SETS][kDims][30];
+    uint32_t shift[SETS][kDims];
+};
+
 // Samples of parent slot `sc` in this round (0: skip the parent).
 __device__ __forceinline__ uint64_t round_samples(const double* sc, int warmup, uint64_t samples)
 {
@@ -97,8 +110,11 @@ __device__ __forceinline__ uint64_t round_samples(const double* sc, int warmup, 
     return warmup ? (uint64_t)sc[kBkWarmup] : samples;
 }
 
-template <typename T, bool SYM>
-__global__ void __launch_bounds__(kThreads) round_kernel(Phys<T> ph, K2Box<T> box, SobolDirsArg dirs,
+// What bounds it: instruction issue (the integrand at one sample per lane, some 500 instructions
+// with the map and the histograms).
+template <typename T, bool SYM, int SETS>
+__global__ void __launch_bounds__(kThreads, (sizeof(T) == 4 ? 4 : 2)) round_kernel(Phys<T> ph, K2Box<T> box,
+                                                         const __grid_constant__ BkDirs<SETS> dirs,
                                                          const double* __restrict__ r_grid, int n,
                                                          const double* __restrict__ spline, const double* state,
                                                          int stride, int bins, int warmup, uint64_t samples,
@@ -117,18 +133,17 @@ __global__ void __launch_bounds__(kThreads) round_kernel(Phys<T> ph, K2Box<T> bo
     int32_t* cnt = reinterpret_cast<int32_t*>(whist + kWarps * kDims * bins);  // [4*bins]
     T* xs = reinterpret_cast<T*>(cnt + kDims * bins + 4);                 // [n] (16-byte aligned)
     T* cs = xs + ((n + 3) & ~3);                                          // [n-1][4] log S block
-    __shared__ uint32_t sst[kDims][30];
-    __shared__ uint32_t ssh[kDims];
+    __shared__ SobolWarp<kDims> sobol;
     __shared__ double red[4][kWarps];
 
+    const int set = SETS == 1 ? 0 : job / n;
     const double* src_coef = spline + n + 4 * (size_t)(n - 1);
     for (int k = threadIdx.x; k < kDims * (bins + 1); k += blockDim.x) edges[k] = st[k];
     for (int k = threadIdx.x; k < kWarps * kDims * bins; k += blockDim.x) whist[k] = 0.0;
     for (int k = threadIdx.x; k < kDims * bins; k += blockDim.x) cnt[k] = 0;
     for (int i = threadIdx.x; i < n; i += blockDim.x) xs[i] = (T)spline[i];
     for (int i = threadIdx.x; i < 4 * (n - 1); i += blockDim.x) cs[i] = (T)src_coef[i];
-    for (int k = threadIdx.x; k < kDims * 30; k += blockDim.x) sst[k / 30][k % 30] = dirs.state[k / 30][k % 30];
-    if (threadIdx.x < kDims) ssh[threadIdx.x] = dirs.shift[threadIdx.x];
+    stage_sobol(sobol, dirs.state[set], dirs.shift[set], bins);
     __syncthreads();
 
     SplineView<T> s;
@@ -139,7 +154,7 @@ __global__ void __launch_bounds__(kThreads) round_kernel(Phys<T> ph, K2Box<T> bo
     s.inv_h = (T)((double)(n - 1) / (spline[n - 1] - spline[0]));
     K2Parent<T> P;
     {
-        const double r = r_grid[job];
+        const double r = r_grid[job - set * n];
         P.r = (T)r;
         P.r2 = P.r * P.r;
         P.lr = (T)log(r);
@@ -151,65 +166,50 @@ __global__ void __launch_bounds__(kThreads) round_kernel(Phys<T> ph, K2Box<T> bo
     const double width[kDims] = {(double)box.width[0], (double)box.width[1], (double)box.width[2],
                                  (double)box.width[3]};
 
-    const uint64_t offset = (uint64_t)sc[kBkOffset];
-    const uint64_t chunk = (total + blocks_per_job - 1) / blocks_per_job;
-    const uint64_t begin = (uint64_t)blockIdx.x * chunk;
-    const uint64_t end = begin + chunk < total ? begin + chunk : total;
+    // this CTA's share of the round's Sobol indices [first, last), in blocks of 32 aligned indices
+    const uint64_t first = (uint64_t)sc[kBkOffset], last = first + total;
+    const uint64_t block0 = first >> 5, blocks = ((last + 31) >> 5) - block0;
+    const uint64_t share = (blocks + blocks_per_job - 1) / blocks_per_job;
+    const uint64_t begin = (uint64_t)blockIdx.x * share;
+    const uint64_t end = begin + share < blocks ? begin + share : blocks;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double* myhist = whist + warp * kDims * bins;
     const double fb = (double)bins;
     double sw = 0.0, sw2 = 0.0, sk2 = 0.0, skf = 0.0;
-    for (uint64_t base = begin; base < end; base += kThreads) {
-        const uint64_t i = base + threadIdx.x;
-        const bool on = i < end;
+    for (uint64_t k = begin + warp; k < end; k += kWarps) {
+        const uint32_t base = (uint32_t)((block0 + k) << 5);
+        const uint64_t index = (uint64_t)base + lane;
+        const bool on = index >= first && index < last;
         int bin[kDims];
-        double w = 0.0, wk2 = 0.0, wkf = 0.0;
-        if (on) {
-            const uint64_t index = offset + i;
-            T x[kDims];
-            double inv_density = 1.0;
+        uint32_t bits[kDims];
+        T x[kDims];
+        double inv_density = 1.0;
 #pragma unroll
-            for (int d = 0; d < kDims; ++d) {
-                const double u = sobol_unit<double>(sobol_bits(sst[d], ssh[d], index), index);
-                const double scaled = u * fb;
-                int b = (int)floor(scaled);
-                b = b > bins - 1 ? bins - 1 : b;
-                const double frac = scaled - b;
-                const double left = edges[d * (bins + 1) + b];
-                const double bw = edges[d * (bins + 1) + b + 1] - left;
-                x[d] = (T)(lower[d] + width[d] * (left + bw * frac));
-                inv_density *= fb * bw;
-                bin[d] = b;
-            }
-            T rec[kRecLen];
-            k2_prepare_x<T>(s, box, x, true, rec);
-            T k2w, kfw;
-            k2_point<T, SYM>(s, ph, P, rec, k2w, kfw);
-            wk2 = (double)k2w * inv_density;
-            wkf = (double)kfw * inv_density;
-            w = ((double)k2w + (double)kfw) * inv_density;
+        for (int d = 0; d < kDims; ++d) {
+            bits[d] = sobol_block_bits(sobol, d, base);
+            double frac;
+            const int b = grid_position(bits[d], bins, frac);
+            const double left = edges[d * (bins + 1) + b];
+            const double bw = edges[d * (bins + 1) + b + 1] - left;
+            x[d] = (T)(lower[d] + width[d] * (left + bw * frac));
+            inv_density *= fb * bw;
+            bin[d] = b;
         }
+        T rec[kRecLen];
+        k2_prepare_x<T>(s, box, x, true, rec);
+        T k2w, kfw;
+        k2_point<T, SYM>(s, ph, P, rec, k2w, kfw);
+        const double w = on ? ((double)k2w + (double)kfw) * inv_density : 0.0;
         sw += w;
         sw2 += w * w;
-        sk2 += wk2;
-        skf += wkf;
-        // deterministic warp histogram: lanes that share a bin add in lane order
-        const unsigned mask = __ballot_sync(0xffffffffu, on);
         if (on) {
-            const double aw = ::fabs(w);
-#pragma unroll
-            for (int d = 0; d < kDims; ++d) {
-                const int key = d * bins + bin[d];
-                const unsigned peers = __match_any_sync(mask, key);
-                const int rank = __popc(peers & ((1u << lane) - 1u));
-                const int last = __reduce_max_sync(mask, rank);
-                for (int k = 0; k <= last; ++k) {
-                    if (rank == k) myhist[key] += aw;
-                    __syncwarp(mask);
-                }
-                atomicAdd(&cnt[key], 1);
-            }
+            sk2 += (double)k2w * inv_density;
+            skf += (double)kfw * inv_density;
         }
+        const double aw = ::fabs(w);
+#pragma unroll
+        for (int d = 0; d < kDims; ++d)
+            warp_hist_add(sobol, d, base, bits[d], on, bin[d], aw, myhist + d * bins, cnt + d * bins);
     }
     for (int o = 16; o > 0; o >>= 1) {
         sw += __shfl_down_sync(0xffffffffu, sw, o);
@@ -245,15 +245,22 @@ __global__ void __launch_bounds__(kThreads) round_kernel(Phys<T> ph, K2Box<T> bo
     }
 }
 
-// Per parent: re-bin the grid from the round's histogram and, for an iteration, fold its
+// Per integral: add the round's partial rows in a fixed order (kSlices interleaved chains per
+// key, then the chains), re-bin the grid from the histogram and, for an iteration, fold its
 // estimate into the weighted combination (value, error, convergence) and the K2 / Kf
 // components; then advance the Sobol offset.
-__global__ void finalize_kernel(double* state, int stride, int bins, int warmup, uint64_t samples,
-                                const double* __restrict__ reduced, int32_t* __restrict__ counts, int min_iterations,
-                                double epsrel, double epsabs)
+constexpr int kFinalThreads = 256;
+
+__global__ void __launch_bounds__(kFinalThreads)
+    finalize_kernel(double* state, int stride, int bins, int warmup, uint64_t samples,
+                    const double* __restrict__ partial, int blocks_per_job, int32_t* __restrict__ counts,
+                    int min_iterations, double epsrel, double epsabs)
 {
     extern __shared__ double fsm[];
-    double* smooth = fsm;                    // [4*bins]
+    const int keys = 4 + kDims * bins;
+    double* red = fsm;                       // [keys]
+    double* chain = red + keys;              // [4][keys], then the re-binning's scratch:
+    double* smooth = chain;                  // [4*bins]
     double* cum = smooth + kDims * bins;     // [4*(bins+1)]
     double* next = cum + kDims * (bins + 1); // [4*(bins+1)]
     const int job = blockIdx.x;
@@ -261,8 +268,22 @@ __global__ void finalize_kernel(double* state, int stride, int bins, int warmup,
     double* sc = st + kDims * (bins + 1);
     const uint64_t n_round = round_samples(sc, warmup, samples);
     if (n_round == 0) return;
-    const int keys = 4 + kDims * bins;
-    const double* red = reduced + (size_t)job * keys;
+    const double* rows = partial + (size_t)job * blocks_per_job * keys;
+    for (int t = threadIdx.x; t < 4 * keys; t += blockDim.x) {
+        const int q = t / keys, k = t - q * keys;
+        double a0 = 0.0, a1 = 0.0;
+        int b = q;
+        for (; b + 4 < blocks_per_job; b += 8) {
+            a0 += rows[(size_t)b * keys + k];
+            a1 += rows[(size_t)(b + 4) * keys + k];
+        }
+        if (b < blocks_per_job) a0 += rows[(size_t)b * keys + k];
+        chain[t] = a0 + a1;
+    }
+    __syncthreads();
+    for (int k = threadIdx.x; k < keys; k += blockDim.x)
+        red[k] = (chain[k] + chain[keys + k]) + (chain[2 * keys + k] + chain[3 * keys + k]);
+    __syncthreads();
     int32_t* c = counts + (size_t)job * kDims * bins;
     rebin(st, red + 2, c, kDims, bins, smooth, cum, next);
     __syncthreads();
@@ -321,16 +342,19 @@ __global__ void replica_select_kernel(const double* __restrict__ N, const double
     }
 }
 
-__global__ void replica_add_kernel(const double* __restrict__ state, int stride, int bins, int points,
+// The sums of `group` replicas (integral = g * points + parent), in replica order.
+__global__ void replica_add_kernel(const double* __restrict__ state, int stride, int bins, int points, int group,
                                    double* __restrict__ acc)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= points) return;
     double* a = acc + (size_t)i * kRepStride;
     if (a[0] == 0.0) return;
-    const double* sc = state + (size_t)i * stride + kDims * (bins + 1);
-    a[1] += sc[kStValue];
-    a[2] += sc[kStError] * sc[kStError];
+    for (int g = 0; g < group; ++g) {
+        const double* sc = state + ((size_t)g * points + i) * stride + kDims * (bins + 1);
+        a[1] += sc[kStValue];
+        a[2] += sc[kStError] * sc[kStError];
+    }
 }
 
 __global__ void replica_end_kernel(const double* __restrict__ acc, int points, int replicas, double* __restrict__ out)
@@ -344,86 +368,129 @@ __global__ void replica_end_kernel(const double* __restrict__ acc, int points, i
     out[3 * i + 2] = a[2] / (m * m);
 }
 
-template <typename T, bool SYM>
-cudaError_t launch_round(const nlo_bk_params& p, const double* r, int points, const double* spline,
-                         const SobolDirsArg& dirs, const nlo_bk_box& box, const BkVegasCall& call, int warmup,
-                         cudaStream_t stream)
+// One round over `group` sets of `points` integrals (the main ones, or a group of replicas).
+struct RoundArgs {
+    const nlo_bk_params& p;
+    const double* r;
+    int points, group;
+    const double* spline;
+    const nlo_bk_box& box;
+    const BkVegasCall& call;
+    double* state;
+    int blocks_per_job;
+    cudaStream_t stream;
+};
+
+template <typename T, bool SYM, int SETS>
+cudaError_t launch_round(const RoundArgs& a, const BkDirs<SETS>& dirs, int warmup)
 {
-    const int bins = call.options.bins;
+    const int bins = a.call.options.bins;
     const size_t smem = sizeof(double) * (kDims * (bins + 1) + kWarps * kDims * bins) +
-                        sizeof(int32_t) * (kDims * bins + 4) + sizeof(T) * (((points + 3) & ~3) + 4 * (points - 1));
-    auto kern = round_kernel<T, SYM>;
+                        sizeof(int32_t) * (kDims * bins + 4) + sizeof(T) * (((a.points + 3) & ~3) + 4 * (a.points - 1));
+    auto kern = round_kernel<T, SYM, SETS>;
     cudaError_t e = raise_dynamic_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     K2Box<T> kb;
     for (int d = 0; d < 4; ++d) {
-        kb.lower[d] = (T)box.lower[d];
-        kb.width[d] = (T)box.width[d];
+        kb.lower[d] = (T)a.box.lower[d];
+        kb.width[d] = (T)a.box.width[d];
     }
-    const double volume = box.width[0] * box.width[1] * box.width[2] * box.width[3];
-    kb.cpt_scale = (T)(volume * p.nc * p.nc / (8.0 * kPi * kPi * kPi * kPi));
-    dim3 grid((unsigned)call.blocks_per_job, (unsigned)points);
-    kern<<<grid, kThreads, smem, stream>>>(make_phys<T>(p), kb, dirs, r, points, spline, call.state,
-                                           call.stride, bins, warmup, (uint64_t)call.options.samples_per_iteration,
-                                           call.blocks_per_job, call.partial, call.counts);
+    const double volume = a.box.width[0] * a.box.width[1] * a.box.width[2] * a.box.width[3];
+    kb.cpt_scale = (T)(volume * a.p.nc * a.p.nc / (8.0 * kPi * kPi * kPi * kPi));
+    dim3 grid((unsigned)a.blocks_per_job, (unsigned)(a.points * a.group));
+    kern<<<grid, kThreads, smem, a.stream>>>(make_phys<T>(a.p), kb, dirs, a.r, a.points, a.spline, a.state,
+                                             a.call.stride, bins, warmup,
+                                             (uint64_t)a.call.options.samples_per_iteration, a.blocks_per_job,
+                                             a.call.partial, a.call.counts);
     return cudaGetLastError();
 }
 
 // The warm-up round (when `with_warmup`) and the iterations of one Vegas call over the
-// parents that `call.state` marks active.
-cudaError_t run_rounds(const nlo_bk_params& p, const double* r, int points, const double* spline,
-                       const SobolDirsArg& dirs, const nlo_bk_box& box, const BkVegasCall& call, bool with_warmup,
-                       cudaStream_t stream)
+// integrals that the state marks active.
+template <int SETS>
+cudaError_t run_rounds(const RoundArgs& a, const BkDirs<SETS>& dirs, bool with_warmup)
 {
-    const nlo_bk_vegas_options& o = call.options;
-    const bool fp64 = p.precision == NLO_PRECISION_FP64;
-    const bool sym = p.symmetrize != 0;
+    const nlo_bk_vegas_options& o = a.call.options;
+    const bool fp64 = a.p.precision == NLO_PRECISION_FP64;
+    const bool sym = a.p.symmetrize != 0;
     const int keys = 4 + kDims * o.bins;
-    const size_t fsmem = sizeof(double) * (kDims * o.bins + 2 * kDims * (o.bins + 1));
+    const size_t fsmem = sizeof(double) * 5 * (size_t)keys;
     cudaError_t e = raise_dynamic_smem((const void*)finalize_kernel, fsmem);
     if (e != cudaSuccess) return e;
     const int rounds = o.max_iterations + (with_warmup ? 1 : 0);
     for (int k = 0; k < rounds; ++k) {
-        const int is_warmup = with_warmup && k == 0;
+        const int warmup = with_warmup && k == 0;
         if (fp64)
-            e = sym ? launch_round<double, true>(p, r, points, spline, dirs, box, call, is_warmup, stream)
-                    : launch_round<double, false>(p, r, points, spline, dirs, box, call, is_warmup, stream);
+            e = sym ? launch_round<double, true>(a, dirs, warmup) : launch_round<double, false>(a, dirs, warmup);
         else
-            e = sym ? launch_round<float, true>(p, r, points, spline, dirs, box, call, is_warmup, stream)
-                    : launch_round<float, false>(p, r, points, spline, dirs, box, call, is_warmup, stream);
+            e = sym ? launch_round<float, true>(a, dirs, warmup) : launch_round<float, false>(a, dirs, warmup);
         if (e != cudaSuccess) return e;
-        if ((e = vegas_launch_reduce(call.partial, keys, call.blocks_per_job, points, call.reduced, stream)) !=
-            cudaSuccess)
-            return e;
-        finalize_kernel<<<points, 128, fsmem, stream>>>(call.state, call.stride, o.bins, is_warmup,
-                                                        (uint64_t)o.samples_per_iteration, call.reduced, call.counts,
-                                                        o.min_iterations, o.epsrel, o.epsabs);
+        finalize_kernel<<<a.points * a.group, kFinalThreads, fsmem, a.stream>>>(
+            a.state, a.call.stride, o.bins, warmup, (uint64_t)o.samples_per_iteration, a.call.partial,
+            a.blocks_per_job, a.call.counts, o.min_iterations, o.epsrel, o.epsabs);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
+template <int SETS>
+BkDirs<SETS> bk_dirs(const SobolDirsArg* dirs, int sets)
+{
+    BkDirs<SETS> b;
+    std::memset(&b, 0, sizeof(b));
+    for (int g = 0; g < sets; ++g) {
+        std::memcpy(b.state[g], dirs[g].state, sizeof(b.state[g]));
+        std::memcpy(b.shift[g], dirs[g].shift, sizeof(b.shift[g]));
+    }
+    return b;
+}
+
+// Integrals of one launch at most: replicas run together up to this many, at least one replica
+// of every parent.
+constexpr int kJobsCap = 4096;
+constexpr int kReplicaSets = 16;  // options.replicas is at most 16
+
 }  // namespace
 
 size_t bk_vegas_state_doubles(int bins) { return (size_t)kDims * (bins + 1) + kStSlots; }
 
-int bk_vegas_blocks_per_job(int points)
+// CTAs per integral: about 2,048 samples each (eight passes of a CTA, enough to outweigh
+// staging its tables: a lone unconverged parent then spreads over 49 SMs at 1e5 samples,
+// where 18 CTAs took 140 us a round), within 16,384 partial rows in all.
+int bk_vegas_blocks_per_job(int points, int64_t samples)
 {
-    int device = 0, sms = 148;
-    if (cudaGetDevice(&device) == cudaSuccess) cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
-    // about two waves of 256-thread CTAs at six per SM over all grid points
-    const int target = 2 * 6 * (sms > 0 ? sms : 148);
-    int b = (target + points - 1) / points;
-    return b < 1 ? 1 : (b > 64 ? 64 : b);
+    const int64_t by_rows = points < 16384 ? 16384 / points : 1;
+    const int64_t want = (samples + 2047) / 2048;
+    const int64_t b = want < by_rows ? want : by_rows;
+    return (int)(b < 1 ? 1 : (b > 64 ? 64 : b));
 }
 
-size_t bk_vegas_scratch_bytes(int points, int bins)
+int bk_vegas_replica_group(int points, int replicas)
 {
-    const size_t keys = 4 + (size_t)kDims * bins;
-    const size_t blocks = (size_t)bk_vegas_blocks_per_job(points);
-    // round partials and sums, bin counts, then the replica grids and accumulators
-    return sizeof(double) * keys * (size_t)points * (blocks + 1) + sizeof(int32_t) * (size_t)kDims * bins * points +
-           256 + sizeof(double) * (bk_vegas_state_doubles(bins) + kRepStride) * (size_t)points + 256;
+    const int fit = kJobsCap / points;
+    const int g = fit < replicas ? fit : replicas;
+    return g < 1 ? 1 : g;
+}
+
+// A replica round has a few parents of each replica: half the CTAs of a main integral.
+static int replica_blocks(int blocks) { return blocks > 1 ? blocks / 2 : 1; }
+
+static size_t partial_rows(int points, const nlo_bk_vegas_options& o)
+{
+    const int64_t most = o.samples_per_iteration > o.warmup_samples ? o.samples_per_iteration : o.warmup_samples;
+    const int blocks = bk_vegas_blocks_per_job(points, most);
+    const size_t main = (size_t)points * blocks;
+    const size_t rep = (size_t)points * bk_vegas_replica_group(points, o.replicas) * replica_blocks(blocks);
+    return o.replicas > 0 && rep > main ? rep : main;
+}
+
+size_t bk_vegas_scratch_bytes(int points, const nlo_bk_vegas_options& o)
+{
+    const size_t keys = 4 + (size_t)kDims * o.bins;
+    const size_t jobs = (size_t)points * bk_vegas_replica_group(points, o.replicas);
+    // round partials, bin counts, then the replica grids and accumulators
+    return sizeof(double) * keys * partial_rows(points, o) + sizeof(int32_t) * (size_t)kDims * o.bins * jobs + 256 +
+           sizeof(double) * (bk_vegas_state_doubles(o.bins) * jobs + kRepStride * (size_t)points) + 256;
 }
 
 BkVegasCall bk_vegas_carve(void* scratch, int points, const nlo_bk_vegas_options& options, double* state)
@@ -432,15 +499,17 @@ BkVegasCall bk_vegas_carve(void* scratch, int points, const nlo_bk_vegas_options
     c.options = options;
     c.state = state;
     c.stride = (int)bk_vegas_state_doubles(options.bins);
-    c.blocks_per_job = bk_vegas_blocks_per_job(points);
+    const int64_t most = options.samples_per_iteration > options.warmup_samples ? options.samples_per_iteration
+                                                                                : options.warmup_samples;
+    c.blocks_per_job = bk_vegas_blocks_per_job(points, most);
     const size_t keys = 4 + (size_t)kDims * options.bins;
+    const size_t jobs = (size_t)points * bk_vegas_replica_group(points, options.replicas);
     char* base = static_cast<char*>(scratch);
     c.partial = reinterpret_cast<double*>(base);
-    c.reduced = c.partial + keys * (size_t)points * (size_t)c.blocks_per_job;
-    c.counts = reinterpret_cast<int32_t*>(c.reduced + keys * (size_t)points);
-    const size_t after = reinterpret_cast<size_t>(c.counts + (size_t)kDims * options.bins * points);
+    c.counts = reinterpret_cast<int32_t*>(c.partial + keys * partial_rows(points, options));
+    const size_t after = reinterpret_cast<size_t>(c.counts + (size_t)kDims * options.bins * jobs);
     c.replica_state = reinterpret_cast<double*>((after + 255) & ~(size_t)255);
-    c.replica_acc = c.replica_state + bk_vegas_state_doubles(options.bins) * (size_t)points;
+    c.replica_acc = c.replica_state + bk_vegas_state_doubles(options.bins) * jobs;
     return c;
 }
 
@@ -461,9 +530,8 @@ cudaError_t launch_k2kf_vegas(const nlo_bk_params& p, const double* r, const dou
                                              o.reuse_grid ? 1 : 0, warmup, reuse_warmup, call.counts, nullptr);
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    if ((e = run_rounds(p, r, points, spline, dirs, box, call, warmup > 0 || reuse_warmup > 0, stream)) !=
-        cudaSuccess)
-        return e;
+    const RoundArgs rounds{p, r, points, 1, spline, box, call, call.state, call.blocks_per_job, stream};
+    if ((e = run_rounds(rounds, bk_dirs<1>(&dirs, 1), warmup > 0 || reuse_warmup > 0)) != cudaSuccess) return e;
     end_kernel<<<(points + 255) / 256, 256, 0, stream>>>(call.state, call.stride, o.bins, points, out);
     return cudaGetLastError();
 }
@@ -478,17 +546,24 @@ cudaError_t launch_k2kf_vegas_refine(const nlo_bk_params& p, const double* r, co
     replica_select_kernel<<<blocks, threads, 0, stream>>>(N, k1, points, call.state, call.stride, o.bins,
                                                           call.replica_acc);
     cudaError_t e = cudaGetLastError();
-    // each replica: a fresh grid with the full warm-up (the reference's new VegasState)
-    BkVegasCall rep = call;
-    rep.state = call.replica_state;
+    // each replica: a fresh grid with the full warm-up (the reference's new VegasState); the
+    // replicas are independent, so a group of them shares its launches (one by one, each left
+    // most SMs idle: a typical right-hand side refines 17 of 92 parents)
     const uint64_t warmup = (uint64_t)o.warmup_samples;
-    for (int k = 0; k < o.replicas && e == cudaSuccess; ++k) {
-        begin_kernel<<<points, 64, 0, stream>>>(N, points, 0, 1, rep.state, rep.stride, o.bins, 0, warmup, 0,
-                                                 rep.counts, call.replica_acc);
+    const int group = bk_vegas_replica_group(points, o.replicas);
+    for (int k = 0; k < o.replicas && e == cudaSuccess; k += group) {
+        const int sets = k + group <= o.replicas ? group : o.replicas - k;
+        begin_kernel<<<points * sets, 64, 0, stream>>>(N, points, 0, 1, call.replica_state, call.stride, o.bins, 0,
+                                                        warmup, 0, call.counts, call.replica_acc);
         if ((e = cudaGetLastError()) != cudaSuccess) break;
-        if ((e = run_rounds(p, r, points, spline, call.replica_dirs[k], box, rep, warmup > 0, stream)) != cudaSuccess)
-            break;
-        replica_add_kernel<<<blocks, threads, 0, stream>>>(rep.state, rep.stride, o.bins, points, call.replica_acc);
+        const RoundArgs rounds{p,    r,
+                               points, sets,
+                               spline, box,
+                               call,   call.replica_state,
+                               replica_blocks(call.blocks_per_job), stream};
+        if ((e = run_rounds(rounds, bk_dirs<kReplicaSets>(call.replica_dirs + k, sets), warmup > 0)) != cudaSuccess) break;
+        replica_add_kernel<<<blocks, threads, 0, stream>>>(call.replica_state, call.stride, o.bins, points, sets,
+                                                           call.replica_acc);
         e = cudaGetLastError();
     }
     if (e != cudaSuccess) return e;

@@ -52,24 +52,36 @@ __device__ inline void rebin(double* edges, const double* hist, const int32_t* c
     if (threadIdx.x < D) {
         const int d = threadIdx.x;
         double* cd = cum + d * (bins + 1);
-        cd[0] = 0.0;
-        for (int b = 0; b < bins; ++b) cd[b + 1] = cd[b] + smooth[d * bins + b];
+        double sum = 0.0;
+        cd[0] = sum;
+#pragma unroll 4
+        for (int b = 0; b < bins; ++b) {
+            sum += smooth[d * bins + b];
+            cd[b + 1] = sum;
+        }
+    }
+    __syncthreads();
+    // every new edge finds its interval by itself (a forward walk of one thread per dimension
+    // was a chain of dependent loads: 17 us for 32 bins, 33 us for 50)
+    for (int t = threadIdx.x; t < D * (bins + 1); t += blockDim.x) {
+        const int d = t / (bins + 1), k = t - d * (bins + 1);
+        const double* cd = cum + d * (bins + 1);
         const double* e = edges + d * (bins + 1);
-        double* out = next + d * (bins + 1);
         const double total = cd[bins];
         const double step = total / bins;
-        int idx = 0;
-        for (int k = 0; k <= bins; ++k) {
-            // torch.linspace(0, total, bins + 1); the targets increase, so the
-            // searchsorted(right) - 1 index only moves forward
-            const double target = k < (bins + 1) / 2 ? step * k : total - step * (bins - k);
-            while (idx < bins && cd[idx + 1] <= target) ++idx;
-            const int i = idx > bins - 1 ? bins - 1 : idx;
-            const double frac = (target - cd[i]) / smooth[d * bins + i];
-            out[k] = e[i] + frac * (e[i + 1] - e[i]);
+        // torch.linspace(0, total, bins + 1); searchsorted(cum, target, right) - 1
+        const double target = k < (bins + 1) / 2 ? step * k : total - step * (bins - k);
+        int lo = 0, hi = bins;  // the number of j in 1..bins with cum[j] <= target
+        while (lo < hi) {
+            const int mid = (lo + hi) >> 1;
+            if (cd[mid + 1] <= target)
+                lo = mid + 1;
+            else
+                hi = mid;
         }
-        out[0] = 0.0;
-        out[bins] = 1.0;
+        const int i = lo > bins - 1 ? bins - 1 : lo;
+        const double frac = (target - cd[i]) / smooth[d * bins + i];
+        next[t] = k == 0 ? 0.0 : k == bins ? 1.0 : e[i] + frac * (e[i + 1] - e[i]);
     }
     __syncthreads();
     for (int k = threadIdx.x; k < D * (bins + 1); k += blockDim.x) edges[k] = next[k];
