@@ -16,6 +16,7 @@
 #include "dis_terms.cuh"
 #include "sobol.cuh"
 #include "vegas_common.cuh"
+#include "vegas_sampling.cuh"
 
 namespace nlo {
 namespace dis {
@@ -320,21 +321,24 @@ __global__ void __launch_bounds__(kVegasThreads, (vegas_min_blocks<T, TERM>())) 
     if (st[D * (bins + 1) + kStConverged] != 0.0) return;  // uniform per job
 
     extern __shared__ __align__(16) unsigned char vsmem[];
-    double* edges = reinterpret_cast<double*>(vsmem);                    // [D][bins+1]
-    double* whist = edges + D * (bins + 1);                              // [warps][D*bins]
+    double2* cells = reinterpret_cast<double2*>(vsmem);                  // [D][bins] left end and width
+    double* whist = reinterpret_cast<double*>(cells + D * bins);         // [warps][D*bins]
     int32_t* cnt = reinterpret_cast<int32_t*>(whist + (kVegasThreads / 32) * D * bins);  // [D*bins]
     __shared__ double red[2][kVegasThreads / 32];
-    __shared__ uint32_t sst[D][30];
-    __shared__ uint32_t ssh[D];
+    __shared__ vegas::SobolWarp<D> sobol;
 
     const int warps = kVegasThreads / 32;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int k = threadIdx.x; k < D * (bins + 1); k += blockDim.x) edges[k] = st[k];
+    const double fb = (double)bins;
+    for (int k = threadIdx.x; k < D * bins; k += blockDim.x) {
+        const int e = k + k / bins;
+        const double left = st[e], width = st[e + 1] - left;
+        cells[k] = make_double2(left, width);
+        cnt[k] = 0;
+    }
     for (int k = threadIdx.x; k < warps * D * bins; k += blockDim.x) whist[k] = 0.0;
-    for (int k = threadIdx.x; k < D * bins; k += blockDim.x) cnt[k] = 0;
     const SobolDirsArg& sd = dirs[job];
-    for (int k = threadIdx.x; k < D * 30; k += blockDim.x) sst[k / 30][k % 30] = sd.state[k / 30][k % 30];
-    if (threadIdx.x < D) ssh[threadIdx.x] = sd.shift[threadIdx.x];
+    vegas::stage_sobol(sobol, sd.state, sd.shift, bins);
     __shared__ __align__(16) unsigned char raw[sizeof(DisArgs<T>)];
     DisArgs<T>& a = *reinterpret_cast<DisArgs<T>*>(raw);
     __shared__ WarpShared<T, TERM, kVegasThreads> ws;
@@ -342,54 +346,38 @@ __global__ void __launch_bounds__(kVegasThreads, (vegas_min_blocks<T, TERM>())) 
     ws.stage(rule);
     __syncthreads();
 
-    const uint64_t chunk = (samples + blocks_per_job - 1) / blocks_per_job;
-    const uint64_t begin = (uint64_t)blockIdx.x * chunk;
-    const uint64_t end = begin + chunk < samples ? begin + chunk : samples;
+    // this CTA's share of the round's Sobol indices [first, last), in blocks of 32 aligned indices
+    const uint64_t first = offset, last = offset + samples;
+    const uint64_t block0 = first >> 5, blocks = ((last + 31) >> 5) - block0;
+    const uint64_t share = (blocks + blocks_per_job - 1) / blocks_per_job;
+    const uint64_t begin = (uint64_t)blockIdx.x * share;
+    const uint64_t end = begin + share < blocks ? begin + share : blocks;
     double tot = 0.0, tot2 = 0.0;
     double* myhist = whist + warp * D * bins;
-    const double fb = (double)bins;
-    for (uint64_t base = begin; base < end; base += kVegasThreads) {
-        const uint64_t i = base + threadIdx.x;
-        const bool active = i < end;
+    for (uint64_t k = begin + warp; k < end; k += warps) {
+        const uint32_t base = (uint32_t)((block0 + k) << 5);
+        const uint64_t index = (uint64_t)base + lane;
+        const bool active = index >= first && index < last;
         double xl[D];
         int bin[D];
+        uint32_t bits[D];
         double inv_density = 1.0;
-        if (active) {
-            const uint64_t index = offset + i;
 #pragma unroll
-            for (int d = 0; d < D; ++d) {
-                const double u = sobol_unit<double>(sobol_bits(sst[d], ssh[d], index), index);
-                const double scaled = u * fb;
-                int b = (int)floor(scaled);
-                b = b > bins - 1 ? bins - 1 : b;
-                const double frac = scaled - b;
-                const double left = edges[d * (bins + 1) + b];
-                const double width = edges[d * (bins + 1) + b + 1] - left;
-                xl[d] = left + width * frac;
-                inv_density *= fb * width;
-                bin[d] = b;
-            }
+        for (int d = 0; d < D; ++d) {
+            bits[d] = vegas::sobol_block_bits(sobol, d, base);
+            double rest;
+            bin[d] = vegas::grid_position(bits[d], bins, rest);
+            const double2 cell = cells[d * bins + bin[d]];
+            xl[d] = cell.x + cell.y * (rest * 9.313225746154785e-10);
+            inv_density *= fb * cell.y;
         }
         const double w = (double)term_value_warp<T, TERM>(a, active, xl, rule, ws) * inv_density;
         tot += w;
         tot2 += w * w;
-        // deterministic warp histogram: lanes that share a bin add in lane order
-        const unsigned mask = __ballot_sync(0xffffffffu, active);
-        if (active) {
-            const double aw = ::fabs(w);
+        const double aw = ::fabs(w);
 #pragma unroll
-            for (int d = 0; d < D; ++d) {
-                const int key = d * bins + bin[d];
-                const unsigned peers = __match_any_sync(mask, key);
-                const int rank = __popc(peers & ((1u << lane) - 1u));
-                const int last = __reduce_max_sync(mask, rank);
-                for (int k = 0; k <= last; ++k) {
-                    if (rank == k) myhist[key] += aw;
-                    __syncwarp(mask);
-                }
-                atomicAdd(&cnt[key], 1);
-            }
-        }
+        for (int d = 0; d < D; ++d)
+            vegas::warp_hist_add(sobol, d, base, bits[d], active, bin[d], aw, myhist + d * bins, cnt + d * bins);
     }
     // block reduction of the sums in warp order
     for (int o = 16; o > 0; o >>= 1) {
@@ -472,10 +460,14 @@ __global__ void vegas_finalize_kernel(double* __restrict__ state, int state_stri
     double* smooth = fsm;               // [D*bins]
     double* cum = smooth + D * bins;    // [D*(bins+1)]
     double* ne = cum + D * (bins + 1);  // [D*(bins+1)]
+    // the scalar slots in shared memory: one trip to L2 instead of one per dependent access
+    __shared__ double sc[kStSlots];
     const int job = blockIdx.x;
     double* st = state + (size_t)job * state_stride;
-    double* sc = st + D * (bins + 1);
+    double* slots = st + D * (bins + 1);
     int32_t* c = counts + (size_t)job * D * bins;
+    if (threadIdx.x < kStSlots) sc[threadIdx.x] = slots[threadIdx.x];
+    __syncthreads();
     if (sc[kStConverged] != 0.0) return;
     const int keys = 2 + D * bins;
     const double* red = reduced + (size_t)job * keys;
@@ -486,6 +478,8 @@ __global__ void vegas_finalize_kernel(double* __restrict__ state, int state_stri
         sc[kStEvals] += (double)samples;
         if (!warmup) vegas::combine(sc, red[0], red[1], (double)samples, min_iterations, epsrel, epsabs);
     }
+    __syncthreads();
+    if (threadIdx.x < kStSlots) slots[threadIdx.x] = sc[threadIdx.x];
 }
 
 __global__ void vegas_init_kernel(double* state, int state_stride, int D, int bins, int jobs, int keep_edges,
@@ -534,8 +528,7 @@ template <typename T, int TERM>
 cudaError_t launch_vegas_round_t(const VegasLaunch& L, cudaStream_t stream)
 {
     constexpr int D = term_dims(TERM);
-    const size_t smem = sizeof(double) * (D * (L.bins + 1) + (kVegasThreads / 32) * D * L.bins) +
-                        sizeof(int32_t) * D * L.bins;
+    const size_t smem = (sizeof(double2) + sizeof(double) * (kVegasThreads / 32) + sizeof(int32_t)) * D * (size_t)L.bins;
     auto kern = vegas_iteration_kernel<T, TERM>;
     cudaError_t e = raise_dynamic_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;

@@ -31,222 +31,6 @@ namespace {
 
 using namespace k2;
 
-// ---------------------------------------------------------------------------
-// FP32 evaluation tuned for instruction count (the kernel is issue-bound).
-// Spline values are carried in log2 units; the log S coefficients are stored
-// pre-scaled to the unit interval, (a, b h, c h^2, d h^3) * log2(e), so that the
-// position u = (log X - x0)/h gives the piece i = floor(u) and t = u - i directly.
-// Amplitudes outside the grid are encoded as p2 = 0 (S = 1, below r_min) and
-// p2 = -150 (S = 0, above r_max), which lets one branch-free difference formula
-// serve every case:  N_A - N_B = S_A (2^(pB-pA) - 1) if pB <= pA, else -S_B (2^(pA-pB) - 1).
-__device__ __forceinline__ float ex2_approx(float x)
-{
-    float y;
-    asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float lg2_approx(float x)
-{
-    float y;
-    asm("lg2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-__device__ __forceinline__ float rcp_approx(float x)
-{
-    float y;
-    asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
-    return y;
-}
-
-
-
-struct FastSpline {
-    // [n + 1] pre-scaled rows (see above): row 0 is (0, 0, 0, 0), the value below r_min
-    // (log2 S = 0, S = 1); rows 1..n-1 are the intervals; row n is (-150, 0, 0, 0), above
-    // r_max (S = 0)
-    const float4* coef;
-    float u_scale;  // (ln 2 / 2) / h : u from log2(X^2)
-    float u_off;    // -x0 / h
-    float u_top;    // n - 1
-};
-
-struct P2S {
-    float p2, S;
-};
-
-
-
-
-struct K2ParentF {
-    float r, r2, lr, two_r, four_r;
-    float alpha_r;  // the RC_NLO = PARENT_NLO coupling
-};
-
-// COUPLING: 0 smooth freeze, 1 smooth freeze capped at alpha_cap, 2 fixed, 3 any coupling
-// of alpha_of_log (flavour thresholds), 4 the parent's coupling (RC_NLO = PARENT_NLO).
-
-// Spline position u = (log X - x0)/h -> (log2 S, S) for a pair of positions.  u is clamped
-// to [-1, n-1]; the row floor(u) + 1 of the table with its two edge rows serves every case
-// (below the grid, inside, above), so there is no edge select.  floor(u) + 1 comes without
-// the XU conversions: u + (2^23 + 1) rounded down holds it in the low mantissa bits.  The
-// clamp, floor and fraction run on the packed instructions, the table lookup and the cubic
-// per component.
-__device__ __forceinline__ void fast_amplitude_pair(const FastSpline& s, f2 u, P2S& ax, P2S& ay)
-{
-    const f2 uc = make_float2(fminf(fmaxf(u.x, -1.0f), s.u_top), fminf(fmaxf(u.y, -1.0f), s.u_top));
-    const f2 shifted = __fadd2_rd(uc, bc2(8388609.0f));  // 2^23 + 1 + floor(uc)
-    const f2 t = sub2(uc, sub2(shifted, bc2(8388609.0f)));
-    const float4 cx = s.coef[__float_as_int(shifted.x) - 0x4B000000];
-    const float4 cy = s.coef[__float_as_int(shifted.y) - 0x4B000000];
-    const float px = fmaf(t.x, fmaf(t.x, fmaf(t.x, cx.w, cx.z), cx.y), cx.x);
-    const float py = fmaf(t.y, fmaf(t.y, fmaf(t.y, cy.w, cy.z), cy.y), cy.x);
-    ax = {px, ex2_approx(px)};
-    ay = {py, ex2_approx(py)};
-}
-
-// ---------------------------------------------------------------------------
-// Two samples per call on the packed FP32x2 pipe of sm_100 (FFMA2/FADD2/FMUL2): the
-// per-evaluation arithmetic of k2_point_fast, component x for sample 2p and y for 2p+1
-// of a pair record (every field of the two samples side by side), so each packed
-// instruction does the work of two.  MUFU operations, compares and selects stay scalar.
-__device__ __forceinline__ f2 rcp2(f2 a) { return make_float2(rcp_approx(a.x), rcp_approx(a.y)); }
-__device__ __forceinline__ f2 lg22(f2 a) { return make_float2(lg2_approx(a.x), lg2_approx(a.y)); }
-__device__ __forceinline__ f2 sel2(bool cx, bool cy, f2 a, f2 b) { return make_float2(cx ? a.x : b.x, cy ? a.y : b.y); }
-
-// N_A - N_B from log2 S values, for a pair
-__device__ __forceinline__ f2 fast_ndiff2(const P2S& Ax, const P2S& Ay, const P2S& Bx, const P2S& By)
-{
-    // N_A - N_B = S_B - S_A.  Near each other (|pB - pA| < 1/2 in log2 units) it is
-    // S_A (2^(pB-pA) - 1) or -S_B (2^(pA-pB) - 1) with 2^x - 1 = x q(x), q a degree-5
-    // polynomial fitted to (2^x - 1)/x on [-1/2, 0] (1.2e-7 relative in FP32); farther
-    // apart the plain difference S_B - S_A has no cancellation (the ratio is at least
-    // sqrt(2)), and both S are at hand.
-    const f2 d = make_float2(Bx.p2 - Ax.p2, By.p2 - Ay.p2);
-    const f2 x = make_float2(-fabsf(d.x), -fabsf(d.y));
-    f2 q = fma2(bc2(0.0001327910803141678f), x, bc2(0.001321632968973654f));
-    q = fma2(q, x, bc2(0.009615099576281485f));
-    q = fma2(q, x, bc2(0.05550375169709732f));
-    q = fma2(q, x, bc2(0.24022649146109623f));
-    q = fma2(q, x, bc2(0.6931471804499034f));
-    const f2 S = make_float2(d.x <= 0.0f ? Ax.S : -Bx.S, d.y <= 0.0f ? Ay.S : -By.S);
-    const f2 near = mul2(S, mul2(q, x));
-    const f2 far = make_float2(Bx.S - Ax.S, By.S - Ay.S);
-    return make_float2(x.x > -0.5f ? near.x : far.x, x.y > -0.5f ? near.y : far.y);
-}
-
-template <bool SYM, int COUPLING>
-__device__ __forceinline__ void k2_pair_fast(const FastSpline& s, const Phys<float>& ph, const K2ParentF& P,
-                                             const float4* __restrict__ rec4, f2& kfw, f2& total)
-{
-    constexpr float LN2 = 0.69314718055994531f;
-    constexpr float L2E = 1.4426950408889634f;
-    // pair layout: float4 k holds fields 2k and 2k+1 of (sample x, sample y)
-    const float4 w0 = rec4[0], w1 = rec4[1], w2 = rec4[2], w3 = rec4[3], w4 = rec4[4];
-    const float4 w5 = rec4[5], w6 = rec4[6], w7 = rec4[7], w8 = rec4[8], w9 = rec4[9];
-    const f2 z = make_float2(w0.x, w0.y), z2 = make_float2(w0.z, w0.w);
-    const f2 s1 = make_float2(w1.x, w1.y), s2 = make_float2(w1.z, w1.w);
-    const f2 P1 = make_float2(w2.x, w2.y), P2 = make_float2(w2.z, w2.w);
-    const f2 U1 = make_float2(w3.x, w3.y), V1 = make_float2(w3.z, w3.w);
-    const f2 U2 = make_float2(w4.x, w4.y), V2 = make_float2(w4.z, w4.w);
-    const f2 q = make_float2(w5.x, w5.y), D1 = make_float2(w5.z, w5.w);
-    const f2 D2 = make_float2(w6.x, w6.y), dN = make_float2(w6.z, w6.w);
-    const f2 SY = make_float2(w7.x, w7.y), Lmin = make_float2(w7.z, w7.w);
-    const f2 cpt = make_float2(w8.x, w8.y), Dl = make_float2(w8.z, w8.w);
-    const f2 zsq = make_float2(w9.x, w9.y), z2sq = make_float2(w9.z, w9.w);
-    const f2 r = bc2(P.r);
-    const f2 rz = sub2(r, z), rz2 = sub2(r, z2);
-    const f2 Xsq = fma2(bc2(P.four_r), s1, mul2(rz, rz));  // s1 = z sin^2(theta/2)
-    const f2 X2sq = fma2(bc2(P.four_r), s2, mul2(rz2, rz2));
-    const f2 L2X = lg22(Xsq), L2X2 = lg22(X2sq);
-    const f2 uX = fma2(L2X, bc2(s.u_scale), bc2(s.u_off)), uX2 = fma2(L2X2, bc2(s.u_scale), bc2(s.u_off));
-    P2S vXx, vXy, vX2x, vX2y;
-    fast_amplitude_pair(s, uX, vXx, vXy);
-    fast_amplitude_pair(s, uX2, vX2x, vX2y);
-    // kernels
-    // log(a/b)/(a - b) = 2 (1 + hm1)/(a + b), hm1 = atanh(t)/t - 1, t = (a - b)/(a + b): the series
-    // in t^2 where |a - b| < (a + b)/2, else log(a/b) directly; each case needs one reciprocal,
-    // of a + b or of a - b, and the test needs none
-    const f2 a = mul2(Xsq, z2sq), b = mul2(X2sq, zsq);
-    const f2 sab = add2(a, b);
-    const f2 d = mul2(r, fma2(r, P1, make_float2(-P2.x, -P2.y)));  // a - b
-    const bool ser_x = fabsf(d.x) < 0.5f * sab.x, ser_y = fabsf(d.y) < 0.5f * sab.y;
-    const f2 rden = rcp2(sel2(ser_x, ser_y, sab, d));
-    const f2 t = mul2(d, rden);
-    const f2 t2 = mul2(t, t);
-    f2 g = fma2(bc2(0.15609439065092748f), t2, bc2(0.04106302733766397f));
-    g = fma2(g, t2, bc2(0.09747851219255123f));
-    g = fma2(g, t2, bc2(0.11051354325642386f));
-    g = fma2(g, t2, bc2(0.1428825580061165f));
-    g = fma2(g, t2, bc2(0.19999959971627077f));
-    g = fma2(g, t2, bc2(0.33333333435159396f));
-    const f2 hm1_series = mul2(g, t2);
-    const f2 Ld = fma2(bc2(LN2), sub2(L2X, L2X2), Dl);  // log(a/b)
-    // log case: 1 + hm1 = log(a/b) (a + b) / (2 (a - b)) and L = log(a/b) / (a - b)
-    const f2 Lr = mul2(Ld, rden);
-    const f2 hm1 = sel2(ser_x, ser_y, hm1_series, fma2(mul2(bc2(0.5f), Lr), sab, bc2(-1.0f)));
-    const f2 rs2 = add2(rden, rden);
-    const f2 L = sel2(ser_x, ser_y, fma2(hm1, rs2, rs2), Lr);
-    const f2 r2Lq = mul2(mul2(bc2(P.r2), L), q);
-    const f2 fq2 = mul2(add2(hm1, hm1), mul2(q, q));
-    const f2 C0 = fma2(bc2(-4.0f), r2Lq, fq2);
-    const f2 B1 = fma2(r, U1, V1), B2 = fma2(r, U2, V2);
-    const f2 w = mul2(r2Lq, bc2(P.two_r));
-    const f2 k2 = fma2(mul2(w, B1), rcp2(mul2(Xsq, z2)), C0);
-    const f2 k2s = fma2(mul2(w, B2), rcp2(mul2(X2sq, z)), C0);
-    const f2 kf = mul2(sub2(r2Lq, fq2), bc2(ph.nf_over_nc));
-    const f2 dip = mul2(make_float2(vXx.S, vXy.S), D1), dips = mul2(make_float2(vX2x.S, vX2y.S), D2);
-    // the cut |K2| > 1e10 with |dipole| < 1e-10 sets both factors to zero: zero their product
-    const bool cut_x = fabsf(k2.x) > 1e10f && fabsf(dip.x) < 1e-10f;
-    const bool cut_y = fabsf(k2.y) > 1e10f && fabsf(dip.y) < 1e-10f;
-    const f2 prod = sel2(cut_x, cut_y, bc2(0.0f), mul2(k2, dip));
-    const f2 dNX = fast_ndiff2(vXx, vXy, vX2x, vX2y);
-    f2 k2part, fermion;
-    if (SYM) {  // the factor 1/2 of the symmetrisation is folded into cpt
-        const bool cuts_x = fabsf(k2s.x) > 1e10f && fabsf(dips.x) < 1e-10f;
-        const bool cuts_y = fabsf(k2s.y) > 1e10f && fabsf(dips.y) < 1e-10f;
-        k2part = add2(prod, sel2(cuts_x, cuts_y, bc2(0.0f), mul2(k2s, dips)));
-        fermion = mul2(mul2(kf, dNX), dN);
-    } else {
-        k2part = prod;
-        fermion = mul2(mul2(kf, SY), dNX);
-    }
-    f2 alpha;
-    if (COUPLING == 2) {
-        alpha = bc2(ph.fixed_as);
-    } else if (COUPLING == 4) {
-        alpha = bc2(P.alpha_r);
-    } else {
-        const f2 lmin = make_float2(fminf(fminf(Lmin.x, P.lr), (0.5f * LN2) * fminf(L2X.x, L2X2.x)),
-                                    fminf(fminf(Lmin.y, P.lr), (0.5f * LN2) * fminf(L2X.y, L2X2.y)));
-        if (COUPLING == 3) {
-            alpha = make_float2(alpha_of_log(lmin.x, ph), alpha_of_log(lmin.y, ph));
-        } else {
-            const f2 right = fma2(bc2(-10.0f), lmin, bc2(5.0f * ph.log_sc));
-            const f2 m = make_float2(fmaxf(ph.left, right.x), fmaxf(ph.left, right.y));
-            const f2 gap = make_float2(fabsf(ph.left - right.x), fabsf(ph.left - right.y));
-            // logaddexp = max + log(1 + e^-gap); beyond gap = 17 the correction is below
-            // 4.2e-8 of max >= 9.16 (FP32 rounding), and the warp skips the two MUFU operations
-            f2 lae = m;
-            if (gap.x < 17.0f || gap.y < 17.0f) {
-                const f2 e = make_float2(ex2_approx(-gap.x * L2E), ex2_approx(-gap.y * L2E));
-                lae = fma2(bc2(LN2), lg22(add2(bc2(1.0f), e)), m);
-            }
-            alpha = rcp2(mul2(bc2(ph.b0c), lae));
-            if (COUPLING == 1) alpha = make_float2(fminf(alpha.x, ph.alpha_cap), fminf(alpha.y, ph.alpha_cap));
-        }
-    }
-    const f2 scale = mul2(mul2(alpha, alpha), cpt);
-    const f2 k2w = mul2(k2part, scale);
-    kfw = mul2(make_float2(-fermion.x, -fermion.y), scale);
-    const f2 tot = add2(k2w, kfw);
-    // X^2 or X'^2 below the normal range (the oracle's validity cut) gives infinite kernels
-    // (the approximate reciprocal flushes denormals), so the finite test covers it
-    const bool ok_x = fabsf(tot.x) < INFINITY;
-    const bool ok_y = fabsf(tot.y) < INFINITY;
-    kfw = sel2(ok_x, ok_y, kfw, bc2(0.0f));
-    total = sel2(ok_x, ok_y, tot, bc2(0.0f));
-}
-
 constexpr int kFoldPairs = 16;
 
 
@@ -610,32 +394,6 @@ cudaError_t launch_typed(const nlo_bk_params& p, const double* r, int points, co
         make_phys<T>(p), make_box<T>(p, box, SYM), dirs, r, points, spline, active, count, offset, samples, partial,
         SetsArg{});
     return cudaGetLastError();
-}
-
-// The kernel instantiation of a parameter set: FP64 (one form for every coupling) or the
-// FP32 coupling variant; f(T(), SYM, COUPLING) with std::integral_constant tags.
-template <class F>
-cudaError_t dispatch_variant(const nlo_bk_params& p, F f)
-{
-    using std::integral_constant;
-    const bool sym = p.symmetrize != 0;
-    const int coupling = p.fixed_coupling                 ? 2
-                         : p.rc_nlo == NLO_RC_NLO_PARENT ? 4
-                         : p.nf > 3.0                    ? 3
-                         : p.alpha_cap > 0.0             ? 1
-                                                         : 0;
-#define NLO_K2_VARIANT(T, C)                                                                  \
-    (sym ? f(T(), integral_constant<bool, true>(), integral_constant<int, C>())                \
-         : f(T(), integral_constant<bool, false>(), integral_constant<int, C>()))
-    if (p.precision == NLO_PRECISION_FP64) return NLO_K2_VARIANT(double, 0);
-    switch (coupling) {
-        case 0: return NLO_K2_VARIANT(float, 0);
-        case 1: return NLO_K2_VARIANT(float, 1);
-        case 2: return NLO_K2_VARIANT(float, 2);
-        case 3: return NLO_K2_VARIANT(float, 3);
-        default: return NLO_K2_VARIANT(float, 4);
-    }
-#undef NLO_K2_VARIANT
 }
 
 // at most 448 lanes (parents) per CTA: the FP32 kernel's bounds (448 threads, two CTAs per

@@ -97,10 +97,10 @@ __global__ void begin_kernel(const double* __restrict__ N, int points, int shard
 
 // Direction numbers of the integrals of one launch: set 0 of the main integrals, set g of the
 // g-th replica (integral / points).
-template <int SETS>
+constexpr int kReplicaSets = 16;  // options.replicas is at most 16
 struct BkDirs {
-    uint32_t state[SETS][kDims][30];
-    uint32_t shift[SETS][kDims];
+    uint32_t state[kReplicaSets][kDims][30];
+    uint32_t shift[kReplicaSets][kDims];
 };
 
 // Samples of parent slot `sc` in this round (0: skip the parent).
@@ -110,11 +110,12 @@ __device__ __forceinline__ uint64_t round_samples(const double* sc, int warmup, 
     return warmup ? (uint64_t)sc[kBkWarmup] : samples;
 }
 
-// What bounds it: instruction issue (the integrand at one sample per lane, some 500 instructions
-// with the map and the histograms).
-template <typename T, bool SYM, int SETS>
-__global__ void __launch_bounds__(kThreads, (sizeof(T) == 4 ? 4 : 2)) round_kernel(Phys<T> ph, K2Box<T> box,
-                                                         const __grid_constant__ BkDirs<SETS> dirs,
+// The FP32 build takes two blocks of 32 samples a pass on the packed FP32x2 instructions, with
+// the QMC kernel's evaluation (k2_pair_fast) and the record formed in registers; FP64 takes one.
+// What bounds it: instruction issue.
+template <typename T, bool SYM, int COUPLING>
+__global__ void __launch_bounds__(kThreads, (sizeof(T) == 4 ? 3 : 2)) round_kernel(Phys<T> ph, K2Box<T> box,
+                                                         const __grid_constant__ BkDirs dirs,
                                                          const double* __restrict__ r_grid, int n,
                                                          const double* __restrict__ spline, const double* state,
                                                          int stride, int bins, int warmup, uint64_t samples,
@@ -127,44 +128,60 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 4 ? 4 : 2)) round_kern
     const uint64_t total = round_samples(sc, warmup, samples);
     if (total == 0) return;  // uniform per CTA
 
+    constexpr bool FAST = sizeof(T) == sizeof(float);
     extern __shared__ __align__(16) unsigned char vsm[];
-    double* edges = reinterpret_cast<double*>(vsm);                       // [4][bins+1]
-    double* whist = edges + kDims * (bins + 1);                           // [warps][4*bins]
+    double2* cells = reinterpret_cast<double2*>(vsm);           // [4][bins] left end and 2^-30 width, box units
+    double* density = reinterpret_cast<double*>(cells + kDims * bins);  // [4][bins] bins x width, unit cube
+    double* whist = density + kDims * bins;                     // [warps][4*bins]
     int32_t* cnt = reinterpret_cast<int32_t*>(whist + kWarps * kDims * bins);  // [4*bins]
-    T* xs = reinterpret_cast<T*>(cnt + kDims * bins + 4);                 // [n] (16-byte aligned)
-    T* cs = xs + ((n + 3) & ~3);                                          // [n-1][4] log S block
+    unsigned char* tables = reinterpret_cast<unsigned char*>(cnt + kDims * bins);  // 16-byte aligned
+    float4* rows = reinterpret_cast<float4*>(tables);           // FP32: [n+1] FastSpline rows
+    double* xs = reinterpret_cast<double*>(tables);             // FP64: knots [n] ...
+    double* cs = xs + ((n + 1) & ~1);                           // ... and the log S block [n-1][4]
     __shared__ SobolWarp<kDims> sobol;
     __shared__ double red[4][kWarps];
 
-    const int set = SETS == 1 ? 0 : job / n;
+    const int set = job / n;
     const double* src_coef = spline + n + 4 * (size_t)(n - 1);
-    for (int k = threadIdx.x; k < kDims * (bins + 1); k += blockDim.x) edges[k] = st[k];
+    const double fb = (double)bins;
+    for (int k = threadIdx.x; k < kDims * bins; k += blockDim.x) {
+        const int d = k / bins, e = k + d;
+        const double left = st[e], width = st[e + 1] - left, span = (double)box.width[d];
+        cells[k] = make_double2((double)box.lower[d] + span * left, span * width * 9.313225746154785e-10);
+        density[k] = fb * width;
+        cnt[k] = 0;
+    }
     for (int k = threadIdx.x; k < kWarps * kDims * bins; k += blockDim.x) whist[k] = 0.0;
-    for (int k = threadIdx.x; k < kDims * bins; k += blockDim.x) cnt[k] = 0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) xs[i] = (T)spline[i];
-    for (int i = threadIdx.x; i < 4 * (n - 1); i += blockDim.x) cs[i] = (T)src_coef[i];
+    const double h = (spline[n - 1] - spline[0]) / (double)(n - 1);
+    if constexpr (FAST) {
+        stage_fast_rows(rows, src_coef, n, h);
+    } else {
+        for (int i = threadIdx.x; i < n; i += blockDim.x) xs[i] = spline[i];
+        for (int i = threadIdx.x; i < 4 * (n - 1); i += blockDim.x) cs[i] = src_coef[i];
+    }
     stage_sobol(sobol, dirs.state[set], dirs.shift[set], bins);
     __syncthreads();
 
-    SplineView<T> s;
-    s.x = xs;
-    s.coef = cs;
-    s.n = n;
-    s.x0 = xs[0];
-    s.inv_h = (T)((double)(n - 1) / (spline[n - 1] - spline[0]));
-    K2Parent<T> P;
-    {
-        const double r = r_grid[job - set * n];
-        P.r = (T)r;
-        P.r2 = P.r * P.r;
-        P.lr = (T)log(r);
-        P.two_r = (T)2 * P.r;
+    const double r = r_grid[job - set * n];
+    FastSpline fs;
+    K2ParentF PF;
+    SplineView<double> s;
+    K2Parent<double> P;
+    if constexpr (FAST) {
+        fs = fast_spline(rows, n, spline[0], h);
+        PF = fast_parent(r, ph);
+    } else {
+        s.x = xs;
+        s.coef = cs;
+        s.n = n;
+        s.x0 = xs[0];
+        s.inv_h = 1.0 / h;
+        P.r = r;
+        P.r2 = r * r;
+        P.lr = log(r);
+        P.two_r = 2.0 * r;
         P.alpha_r = alpha_of_log(P.lr, ph);
     }
-    const double lower[kDims] = {(double)box.lower[0], (double)box.lower[1], (double)box.lower[2],
-                                 (double)box.lower[3]};
-    const double width[kDims] = {(double)box.width[0], (double)box.width[1], (double)box.width[2],
-                                 (double)box.width[3]};
 
     // this CTA's share of the round's Sobol indices [first, last), in blocks of 32 aligned indices
     const uint64_t first = (uint64_t)sc[kBkOffset], last = first + total;
@@ -174,42 +191,62 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 4 ? 4 : 2)) round_kern
     const uint64_t end = begin + share < blocks ? begin + share : blocks;
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double* myhist = whist + warp * kDims * bins;
-    const double fb = (double)bins;
     double sw = 0.0, sw2 = 0.0, sk2 = 0.0, skf = 0.0;
-    for (uint64_t k = begin + warp; k < end; k += kWarps) {
-        const uint32_t base = (uint32_t)((block0 + k) << 5);
-        const uint64_t index = (uint64_t)base + lane;
-        const bool on = index >= first && index < last;
+    // a block's point of this lane: box position, weight factor, where it falls
+    struct Sample {
+        uint32_t base, bits[kDims];
         int bin[kDims];
-        uint32_t bits[kDims];
         T x[kDims];
-        double inv_density = 1.0;
+        double factor;
+        bool on;
+    };
+    auto sample = [&](uint64_t k, Sample& p) {
+        p.base = (uint32_t)((block0 + k) << 5);
+        const uint64_t index = (uint64_t)p.base + lane;
+        p.on = k < end && index >= first && index < last;
+        p.factor = 1.0;
 #pragma unroll
         for (int d = 0; d < kDims; ++d) {
-            bits[d] = sobol_block_bits(sobol, d, base);
-            double frac;
-            const int b = grid_position(bits[d], bins, frac);
-            const double left = edges[d * (bins + 1) + b];
-            const double bw = edges[d * (bins + 1) + b + 1] - left;
-            x[d] = (T)(lower[d] + width[d] * (left + bw * frac));
-            inv_density *= fb * bw;
-            bin[d] = b;
+            p.bits[d] = sobol_block_bits(sobol, d, p.base);
+            double rest;
+            p.bin[d] = grid_position(p.bits[d], bins, rest);
+            const double2 cell = cells[d * bins + p.bin[d]];
+            p.x[d] = (T)fma(rest, cell.y, cell.x);
+            p.factor *= density[d * bins + p.bin[d]];
         }
-        T rec[kRecLen];
-        k2_prepare_x<T>(s, box, x, true, rec);
-        T k2w, kfw;
-        k2_point<T, SYM>(s, ph, P, rec, k2w, kfw);
-        const double w = on ? ((double)k2w + (double)kfw) * inv_density : 0.0;
+    };
+    auto record = [&](const Sample& p, double total_w, double kf_w) {
+        // a lane without a sample adds zeros and no counts
+        const double w = p.on ? total_w * p.factor : 0.0, wkf = p.on ? kf_w * p.factor : 0.0;
         sw += w;
         sw2 += w * w;
-        if (on) {
-            sk2 += (double)k2w * inv_density;
-            skf += (double)kfw * inv_density;
-        }
+        sk2 += w - wkf;
+        skf += wkf;
         const double aw = ::fabs(w);
 #pragma unroll
         for (int d = 0; d < kDims; ++d)
-            warp_hist_add(sobol, d, base, bits[d], on, bin[d], aw, myhist + d * bins, cnt + d * bins);
+            warp_hist_add(sobol, d, p.base, p.bits[d], p.on, p.bin[d], aw, myhist + d * bins, cnt + d * bins);
+    };
+    for (uint64_t k = begin + warp; k < end; k += FAST ? 2 * kWarps : kWarps) {
+        Sample a;
+        sample(k, a);
+        if constexpr (FAST) {
+            Sample b;
+            sample(k + kWarps, b);
+            float4 rec4[kRecLen / 2];
+            k2_prepare_pair(fs, box.cpt_scale, make_float2(a.x[0], b.x[0]), make_float2(a.x[1], b.x[1]),
+                            make_float2(a.x[2], b.x[2]), make_float2(a.x[3], b.x[3]), rec4);
+            f2 kf, tot;
+            k2_pair_fast<SYM, COUPLING>(fs, ph, PF, rec4, kf, tot);
+            record(a, (double)tot.x, (double)kf.x);
+            record(b, (double)tot.y, (double)kf.y);
+        } else {
+            T rec[kRecLen];
+            k2_prepare_x<T>(s, box, a.x, true, rec);
+            T k2w, kfw;
+            k2_point<T, SYM>(s, ph, P, rec, k2w, kfw);
+            record(a, k2w + kfw, kfw);
+        }
     }
     for (int o = 16; o > 0; o >>= 1) {
         sw += __shfl_down_sync(0xffffffffu, sw, o);
@@ -263,9 +300,13 @@ __global__ void __launch_bounds__(kFinalThreads)
     double* smooth = chain;                  // [4*bins]
     double* cum = smooth + kDims * bins;     // [4*(bins+1)]
     double* next = cum + kDims * (bins + 1); // [4*(bins+1)]
+    // the scalar slots in shared memory: one trip to L2 instead of one per dependent access
+    __shared__ double sc[kStSlots];
     const int job = blockIdx.x;
     double* st = state + (size_t)job * stride;
-    double* sc = st + kDims * (bins + 1);
+    double* slots = st + kDims * (bins + 1);
+    if (threadIdx.x < kStSlots) sc[threadIdx.x] = slots[threadIdx.x];
+    __syncthreads();
     const uint64_t n_round = round_samples(sc, warmup, samples);
     if (n_round == 0) return;
     const double* rows = partial + (size_t)job * blocks_per_job * keys;
@@ -299,6 +340,8 @@ __global__ void __launch_bounds__(kFinalThreads)
         sc[kBkOffset] += n;
         sc[kBkHasGrid] = 1.0;
     }
+    __syncthreads();
+    if (threadIdx.x < kStSlots) slots[threadIdx.x] = sc[threadIdx.x];
 }
 
 // The right-hand side's K2+Kf per parent in the layout of nlo_bk_k2kf's sums: [value, 0,
@@ -368,6 +411,17 @@ __global__ void replica_end_kernel(const double* __restrict__ acc, int points, i
     out[3 * i + 2] = a[2] / (m * m);
 }
 
+// CTAs per integral: about 2,048 samples each (eight passes of a CTA, enough to outweigh
+// staging its tables: a lone unconverged parent then spreads over 49 SMs at 1e5 samples,
+// where 18 CTAs took 140 us a round), within 16,384 partial rows in all.
+int bk_vegas_blocks_per_job(int points, int64_t samples)
+{
+    const int64_t by_rows = points < 16384 ? 16384 / points : 1;
+    const int64_t want = (samples + 2047) / 2048;
+    const int64_t b = want < by_rows ? want : by_rows;
+    return (int)(b < 1 ? 1 : (b > 64 ? 64 : b));
+}
+
 // One round over `group` sets of `points` integrals (the main ones, or a group of replicas).
 struct RoundArgs {
     const nlo_bk_params& p;
@@ -381,13 +435,14 @@ struct RoundArgs {
     cudaStream_t stream;
 };
 
-template <typename T, bool SYM, int SETS>
-cudaError_t launch_round(const RoundArgs& a, const BkDirs<SETS>& dirs, int warmup)
+template <typename T, bool SYM, int COUPLING>
+cudaError_t launch_round(const RoundArgs& a, const BkDirs& dirs, int warmup, int blocks)
 {
     const int bins = a.call.options.bins;
-    const size_t smem = sizeof(double) * (kDims * (bins + 1) + kWarps * kDims * bins) +
-                        sizeof(int32_t) * (kDims * bins + 4) + sizeof(T) * (((a.points + 3) & ~3) + 4 * (a.points - 1));
-    auto kern = round_kernel<T, SYM, SETS>;
+    const size_t tables = sizeof(T) == sizeof(float) ? sizeof(float4) * (size_t)(a.points + 1)
+                                                     : sizeof(double) * (size_t)(((a.points + 1) & ~1) + 4 * (a.points - 1));
+    const size_t smem = (sizeof(double2) + sizeof(double) * (1 + kWarps) + sizeof(int32_t)) * kDims * (size_t)bins + tables;
+    auto kern = round_kernel<T, SYM, COUPLING>;
     cudaError_t e = raise_dynamic_smem((const void*)kern, smem);
     if (e != cudaSuccess) return e;
     K2Box<T> kb;
@@ -396,23 +451,28 @@ cudaError_t launch_round(const RoundArgs& a, const BkDirs<SETS>& dirs, int warmu
         kb.width[d] = (T)a.box.width[d];
     }
     const double volume = a.box.width[0] * a.box.width[1] * a.box.width[2] * a.box.width[3];
-    kb.cpt_scale = (T)(volume * a.p.nc * a.p.nc / (8.0 * kPi * kPi * kPi * kPi));
-    dim3 grid((unsigned)a.blocks_per_job, (unsigned)(a.points * a.group));
+    // k2_pair_fast expects the symmetrisation's 1/2 in the weight
+    const double half = sizeof(T) == sizeof(float) && SYM ? 0.5 : 1.0;
+    kb.cpt_scale = (T)(half * volume * a.p.nc * a.p.nc / (8.0 * kPi * kPi * kPi * kPi));
+    dim3 grid((unsigned)blocks, (unsigned)(a.points * a.group));
     kern<<<grid, kThreads, smem, a.stream>>>(make_phys<T>(a.p), kb, dirs, a.r, a.points, a.spline, a.state,
                                              a.call.stride, bins, warmup,
-                                             (uint64_t)a.call.options.samples_per_iteration, a.blocks_per_job,
-                                             a.call.partial, a.call.counts);
+                                             (uint64_t)a.call.options.samples_per_iteration, blocks, a.call.partial,
+                                             a.call.counts);
     return cudaGetLastError();
 }
 
 // The warm-up round (when `with_warmup`) and the iterations of one Vegas call over the
-// integrals that the state marks active.
-template <int SETS>
-cudaError_t run_rounds(const RoundArgs& a, const BkDirs<SETS>& dirs, bool with_warmup)
+// integrals that the state marks active; `dirs`: the direction numbers of the a.group sets.
+cudaError_t run_rounds(const RoundArgs& a, const SobolDirsArg* dirs, bool with_warmup)
 {
     const nlo_bk_vegas_options& o = a.call.options;
-    const bool fp64 = a.p.precision == NLO_PRECISION_FP64;
-    const bool sym = a.p.symmetrize != 0;
+    BkDirs sets;
+    std::memset(&sets, 0, sizeof(sets));
+    for (int g = 0; g < a.group; ++g) {
+        std::memcpy(sets.state[g], dirs[g].state, sizeof(sets.state[g]));
+        std::memcpy(sets.shift[g], dirs[g].shift, sizeof(sets.shift[g]));
+    }
     const int keys = 4 + kDims * o.bins;
     const size_t fsmem = sizeof(double) * 5 * (size_t)keys;
     cudaError_t e = raise_dynamic_smem((const void*)finalize_kernel, fsmem);
@@ -420,50 +480,28 @@ cudaError_t run_rounds(const RoundArgs& a, const BkDirs<SETS>& dirs, bool with_w
     const int rounds = o.max_iterations + (with_warmup ? 1 : 0);
     for (int k = 0; k < rounds; ++k) {
         const int warmup = with_warmup && k == 0;
-        if (fp64)
-            e = sym ? launch_round<double, true>(a, dirs, warmup) : launch_round<double, false>(a, dirs, warmup);
-        else
-            e = sym ? launch_round<float, true>(a, dirs, warmup) : launch_round<float, false>(a, dirs, warmup);
+        // a round of fewer samples (the warm-up) takes fewer CTAs per integral
+        const int64_t n = warmup ? o.warmup_samples : o.samples_per_iteration;
+        const int wanted = bk_vegas_blocks_per_job(a.points, n);
+        const int blocks = wanted < a.blocks_per_job ? wanted : a.blocks_per_job;
+        e = dispatch_variant(a.p, [&](auto t, auto sym, auto c) {
+            return launch_round<decltype(t), decltype(sym)::value, decltype(c)::value>(a, sets, warmup, blocks);
+        });
         if (e != cudaSuccess) return e;
         finalize_kernel<<<a.points * a.group, kFinalThreads, fsmem, a.stream>>>(
-            a.state, a.call.stride, o.bins, warmup, (uint64_t)o.samples_per_iteration, a.call.partial,
-            a.blocks_per_job, a.call.counts, o.min_iterations, o.epsrel, o.epsabs);
+            a.state, a.call.stride, o.bins, warmup, (uint64_t)o.samples_per_iteration, a.call.partial, blocks,
+            a.call.counts, o.min_iterations, o.epsrel, o.epsabs);
         if ((e = cudaGetLastError()) != cudaSuccess) return e;
     }
     return cudaSuccess;
 }
 
-template <int SETS>
-BkDirs<SETS> bk_dirs(const SobolDirsArg* dirs, int sets)
-{
-    BkDirs<SETS> b;
-    std::memset(&b, 0, sizeof(b));
-    for (int g = 0; g < sets; ++g) {
-        std::memcpy(b.state[g], dirs[g].state, sizeof(b.state[g]));
-        std::memcpy(b.shift[g], dirs[g].shift, sizeof(b.shift[g]));
-    }
-    return b;
-}
-
 // Integrals of one launch at most: replicas run together up to this many, at least one replica
 // of every parent.
 constexpr int kJobsCap = 4096;
-constexpr int kReplicaSets = 16;  // options.replicas is at most 16
-
 }  // namespace
 
 size_t bk_vegas_state_doubles(int bins) { return (size_t)kDims * (bins + 1) + kStSlots; }
-
-// CTAs per integral: about 2,048 samples each (eight passes of a CTA, enough to outweigh
-// staging its tables: a lone unconverged parent then spreads over 49 SMs at 1e5 samples,
-// where 18 CTAs took 140 us a round), within 16,384 partial rows in all.
-int bk_vegas_blocks_per_job(int points, int64_t samples)
-{
-    const int64_t by_rows = points < 16384 ? 16384 / points : 1;
-    const int64_t want = (samples + 2047) / 2048;
-    const int64_t b = want < by_rows ? want : by_rows;
-    return (int)(b < 1 ? 1 : (b > 64 ? 64 : b));
-}
 
 int bk_vegas_replica_group(int points, int replicas)
 {
@@ -531,7 +569,7 @@ cudaError_t launch_k2kf_vegas(const nlo_bk_params& p, const double* r, const dou
     cudaError_t e = cudaGetLastError();
     if (e != cudaSuccess) return e;
     const RoundArgs rounds{p, r, points, 1, spline, box, call, call.state, call.blocks_per_job, stream};
-    if ((e = run_rounds(rounds, bk_dirs<1>(&dirs, 1), warmup > 0 || reuse_warmup > 0)) != cudaSuccess) return e;
+    if ((e = run_rounds(rounds, &dirs, warmup > 0 || reuse_warmup > 0)) != cudaSuccess) return e;
     end_kernel<<<(points + 255) / 256, 256, 0, stream>>>(call.state, call.stride, o.bins, points, out);
     return cudaGetLastError();
 }
@@ -561,7 +599,7 @@ cudaError_t launch_k2kf_vegas_refine(const nlo_bk_params& p, const double* r, co
                                spline, box,
                                call,   call.replica_state,
                                replica_blocks(call.blocks_per_job), stream};
-        if ((e = run_rounds(rounds, bk_dirs<kReplicaSets>(call.replica_dirs + k, sets), warmup > 0)) != cudaSuccess) break;
+        if ((e = run_rounds(rounds, call.replica_dirs + k, warmup > 0)) != cudaSuccess) break;
         replica_add_kernel<<<blocks, threads, 0, stream>>>(call.replica_state, call.stride, o.bins, points, sets,
                                                            call.replica_acc);
         e = cudaGetLastError();

@@ -63,8 +63,8 @@ __device__ __forceinline__ uint32_t sobol_block_bits(const SobolWarp<D>& s, int 
     return base + lane == 0 ? (uint32_t)__uint2float_rn(bits) : bits;
 }
 
-// Position of a coordinate in the grid: bin and fraction of u = bits 2^-30 (the products are
-// exact, as in FP64).
+// Position of a coordinate u = bits 2^-30 in the grid: its bin, and 2^30 times the fraction within
+// it (both exact).
 __device__ __forceinline__ int grid_position(uint32_t bits, int bins, double& frac)
 {
     const uint64_t scaled = (uint64_t)bits * (uint32_t)bins;
@@ -72,7 +72,7 @@ __device__ __forceinline__ int grid_position(uint32_t bits, int bins, double& fr
     b = b > bins - 1 ? bins - 1 : b;
     const uint32_t rest = (uint32_t)(scaled - ((uint64_t)b << 30));
     // rest <= 2^30: 2^52 + rest holds it exactly
-    frac = (__hiloint2double(0x43300000, (int)rest) - 4503599627370496.0) * 9.313225746154785e-10;
+    frac = __hiloint2double(0x43300000, (int)rest) - 4503599627370496.0;
     return b;
 }
 
