@@ -353,6 +353,7 @@ __global__ void __launch_bounds__(kVegasThreads, (vegas_min_blocks<T, TERM>())) 
     const uint64_t begin = (uint64_t)blockIdx.x * share;
     const uint64_t end = begin + share < blocks ? begin + share : blocks;
     double tot = 0.0, tot2 = 0.0;
+    int whole = 0;
     double* myhist = whist + warp * D * bins;
     for (uint64_t k = begin + warp; k < end; k += warps) {
         const uint32_t base = (uint32_t)((block0 + k) << 5);
@@ -375,10 +376,9 @@ __global__ void __launch_bounds__(kVegasThreads, (vegas_min_blocks<T, TERM>())) 
         tot += w;
         tot2 += w * w;
         const double aw = ::fabs(w);
-#pragma unroll
-        for (int d = 0; d < D; ++d)
-            vegas::warp_hist_add(sobol, d, base, bits[d], active, bin[d], aw, myhist + d * bins, cnt + d * bins);
+        vegas::warp_hist_add(sobol, base, bits, active, bin, bins, aw, myhist, cnt, whole);
     }
+    vegas::add_whole_blocks<D>(whole, cnt);
     // block reduction of the sums in warp order
     for (int o = 16; o > 0; o >>= 1) {
         tot += __shfl_down_sync(0xffffffffu, tot, o);
@@ -471,13 +471,14 @@ __global__ void vegas_finalize_kernel(double* __restrict__ state, int state_stri
     if (sc[kStConverged] != 0.0) return;
     const int keys = 2 + D * bins;
     const double* red = reduced + (size_t)job * keys;
-    vegas::rebin(st, red + 2, c, D, bins, smooth, cum, ne);
-    __syncthreads();
-    for (int k = threadIdx.x; k < D * bins; k += blockDim.x) c[k] = 0;
-    if (threadIdx.x == 0) {
+    // the last thread's chain of divisions runs beside the re-binning
+    if (threadIdx.x == blockDim.x - 1) {
         sc[kStEvals] += (double)samples;
         if (!warmup) vegas::combine(sc, red[0], red[1], (double)samples, min_iterations, epsrel, epsabs);
     }
+    vegas::rebin(st, red + 2, c, D, bins, smooth, cum, ne);
+    __syncthreads();
+    for (int k = threadIdx.x; k < D * bins; k += blockDim.x) c[k] = 0;
     __syncthreads();
     if (threadIdx.x < kStSlots) slots[threadIdx.x] = sc[threadIdx.x];
 }
@@ -547,7 +548,7 @@ cudaError_t launch_vegas_round_t(const VegasLaunch& L, cudaStream_t stream)
     const size_t fsmem = sizeof(double) * (D * L.bins + 2 * D * (L.bins + 1));
     e = raise_dynamic_smem((const void*)vegas_finalize_kernel, fsmem);
     if (e != cudaSuccess) return e;
-    vegas_finalize_kernel<<<L.jobs, 128, fsmem, stream>>>(L.state, L.state_stride, D, L.bins, L.samples, L.reduced,
+    vegas_finalize_kernel<<<L.jobs, 256, fsmem, stream>>>(L.state, L.state_stride, D, L.bins, L.samples, L.reduced,
                                                           L.counts, L.warmup, L.min_iterations, L.epsrel, L.epsabs);
     return cudaGetLastError();
 }
@@ -665,7 +666,7 @@ cudaError_t dis_launch_reduce_finalize(int D, int bins, int jobs, int blocks_per
     const size_t fsmem = sizeof(double) * (D * bins + 2 * D * (bins + 1));
     e = raise_dynamic_smem((const void*)dis::vegas_finalize_kernel, fsmem);
     if (e != cudaSuccess) return e;
-    dis::vegas_finalize_kernel<<<jobs, 128, fsmem, stream>>>(state, state_stride, D, bins, samples, reduced, counts,
+    dis::vegas_finalize_kernel<<<jobs, 256, fsmem, stream>>>(state, state_stride, D, bins, samples, reduced, counts,
                                                                warmup, min_iterations, epsrel, epsabs);
     return cudaGetLastError();
 }

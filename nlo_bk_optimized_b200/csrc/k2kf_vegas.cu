@@ -192,6 +192,7 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 4 ? 3 : 2)) round_kern
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     double* myhist = whist + warp * kDims * bins;
     double sw = 0.0, sw2 = 0.0, sk2 = 0.0, skf = 0.0;
+    int whole = 0;
     // a block's point of this lane: box position, weight factor, where it falls
     struct Sample {
         uint32_t base, bits[kDims];
@@ -223,9 +224,7 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 4 ? 3 : 2)) round_kern
         sk2 += w - wkf;
         skf += wkf;
         const double aw = ::fabs(w);
-#pragma unroll
-        for (int d = 0; d < kDims; ++d)
-            warp_hist_add(sobol, d, p.base, p.bits[d], p.on, p.bin[d], aw, myhist + d * bins, cnt + d * bins);
+        warp_hist_add(sobol, p.base, p.bits, p.on, p.bin, bins, aw, myhist, cnt, whole);
     };
     for (uint64_t k = begin + warp; k < end; k += FAST ? 2 * kWarps : kWarps) {
         Sample a;
@@ -248,6 +247,7 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 4 ? 3 : 2)) round_kern
             record(a, k2w + kfw, kfw);
         }
     }
+    add_whole_blocks<kDims>(whole, cnt);
     for (int o = 16; o > 0; o >>= 1) {
         sw += __shfl_down_sync(0xffffffffu, sw, o);
         sw2 += __shfl_down_sync(0xffffffffu, sw2, o);
@@ -286,7 +286,7 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 4 ? 3 : 2)) round_kern
 // key, then the chains), re-bin the grid from the histogram and, for an iteration, fold its
 // estimate into the weighted combination (value, error, convergence) and the K2 / Kf
 // components; then advance the Sobol offset.
-constexpr int kFinalThreads = 256;
+constexpr int kFinalThreads = 544;  // 4 x (4 + 4 x 32) sums at the default 32 bins
 
 __global__ void __launch_bounds__(kFinalThreads)
     finalize_kernel(double* state, int stride, int bins, int warmup, uint64_t samples,
@@ -312,24 +312,18 @@ __global__ void __launch_bounds__(kFinalThreads)
     const double* rows = partial + (size_t)job * blocks_per_job * keys;
     for (int t = threadIdx.x; t < 4 * keys; t += blockDim.x) {
         const int q = t / keys, k = t - q * keys;
-        double a0 = 0.0, a1 = 0.0;
-        int b = q;
-        for (; b + 4 < blocks_per_job; b += 8) {
-            a0 += rows[(size_t)b * keys + k];
-            a1 += rows[(size_t)(b + 4) * keys + k];
-        }
-        if (b < blocks_per_job) a0 += rows[(size_t)b * keys + k];
-        chain[t] = a0 + a1;
+        double sum = 0.0;
+#pragma unroll 8
+        for (int b = q; b < blocks_per_job; b += 4) sum += rows[(size_t)b * keys + k];
+        chain[t] = sum;
     }
     __syncthreads();
     for (int k = threadIdx.x; k < keys; k += blockDim.x)
         red[k] = (chain[k] + chain[keys + k]) + (chain[2 * keys + k] + chain[3 * keys + k]);
     __syncthreads();
     int32_t* c = counts + (size_t)job * kDims * bins;
-    rebin(st, red + 2, c, kDims, bins, smooth, cum, next);
-    __syncthreads();
-    for (int k = threadIdx.x; k < kDims * bins; k += blockDim.x) c[k] = 0;
-    if (threadIdx.x == 0) {
+    // the last thread's chain of divisions runs beside the re-binning
+    if (threadIdx.x == blockDim.x - 1) {
         const double n = (double)n_round;
         sc[kStEvals] += n;
         if (!warmup) {
@@ -340,6 +334,9 @@ __global__ void __launch_bounds__(kFinalThreads)
         sc[kBkOffset] += n;
         sc[kBkHasGrid] = 1.0;
     }
+    rebin(st, red + 2, c, kDims, bins, smooth, cum, next);
+    __syncthreads();
+    for (int k = threadIdx.x; k < kDims * bins; k += blockDim.x) c[k] = 0;
     __syncthreads();
     if (threadIdx.x < kStSlots) slots[threadIdx.x] = sc[threadIdx.x];
 }

@@ -28,14 +28,18 @@ template <int D>
 struct SobolWarp {
     uint32_t dir[D][32], low[D][32], shift[D];
     int phases[D];
+    bool even;  // 32 bins and a net in every dimension: a whole block counts once in every bin
 };
 
-// `state` and `shift` as in nlo_sobol_dirs; called by all threads, before a barrier.
+// `state` and `shift` as in nlo_sobol_dirs; called by all threads of the CTA, before a
+// barrier.
 template <int D>
 __device__ __forceinline__ void stage_sobol(SobolWarp<D>& s, const uint32_t (*state)[30], const uint32_t* shift,
                                             int bins)
 {
     const int lane = threadIdx.x & 31, warps = blockDim.x >> 5;
+    if (threadIdx.x == 0) s.even = bins == 32;
+    __syncthreads();
     for (int d = threadIdx.x >> 5; d < D; d += warps) {
         s.dir[d][lane] = lane < 30 ? state[d][lane] : 0u;
         const uint32_t g = lane ^ (lane >> 1);
@@ -47,6 +51,7 @@ __device__ __forceinline__ void stage_sobol(SobolWarp<D>& s, const uint32_t (*st
         if (lane == 0) {
             s.shift[d] = shift[d];
             s.phases[d] = !net ? 32 : bins % 32 == 0 ? 1 : (bins + 31) / bins + 1;
+            if (!net) s.even = false;
         }
     }
 }
@@ -59,8 +64,9 @@ __device__ __forceinline__ uint32_t sobol_block_bits(const SobolWarp<D>& s, int 
     const int lane = threadIdx.x & 31;
     const uint32_t g = base ^ (base >> 1);
     const uint32_t block = __reduce_xor_sync(0xffffffffu, (g >> lane) & 1u ? s.dir[d][lane] : 0u);
-    const uint32_t bits = block ^ s.shift[d] ^ s.low[d][lane];
-    return base + lane == 0 ? (uint32_t)__uint2float_rn(bits) : bits;
+    uint32_t bits = block ^ s.shift[d] ^ s.low[d][lane];
+    if (base == 0 && lane == 0) bits = (uint32_t)__uint2float_rn(bits);
+    return bits;
 }
 
 // Position of a coordinate u = bits 2^-30 in the grid: its bin, and 2^30 times the fraction within
@@ -76,25 +82,41 @@ __device__ __forceinline__ int grid_position(uint32_t bits, int bins, double& fr
     return b;
 }
 
-// hist[bin] += value and count[bin] += 1 of the active lanes, `hist` the warp's own row.  All
-// lanes call it; `bits` tells the lane's interval of length 1/32.
-// The caller's warps synchronise before they read the row (a barrier of the CTA).
+// hist[bin] += value of the active lanes in every dimension, `hist` the warp's own rows
+// [D][bins], and count[bin] += 1 in the CTA's; a whole block of an even grid only adds to `whole`,
+// for add_whole_blocks.  All lanes call it; bits tell a lane's intervals of length 1/32.  The
+// caller synchronises the CTA before the rows are read.
 template <int D>
-__device__ __forceinline__ void warp_hist_add(const SobolWarp<D>& s, int d, uint32_t base, uint32_t bits, bool active,
-                                              int bin, double value, double* hist, int32_t* count)
+__device__ __forceinline__ void warp_hist_add(const SobolWarp<D>& s, uint32_t base, const uint32_t (&bits)[D],
+                                              bool active, const int (&bin)[D], int bins, double value, double* hist,
+                                              int32_t* count, int& whole)
 {
-    const int phases = base == 0 ? 32 : s.phases[d];
-    const int interval = (int)(bits >> 25);
-    if (phases == 1) {
-        if (active) hist[bin] += value;
-    } else {
-        const int mine = phases == 2 ? interval & 1 : phases == 32 ? (int)(threadIdx.x & 31) : interval % phases;
-        for (int p = 0; p < phases; ++p) {
-            if (active && mine == p) hist[bin] += value;
-            __syncwarp();
+    const bool counted = s.even && base != 0 && __all_sync(0xffffffffu, active);
+    if (counted) ++whole;
+#pragma unroll
+    for (int d = 0; d < D; ++d) {
+        const int phases = base == 0 ? 32 : s.phases[d];
+        const int interval = (int)(bits[d] >> 25);
+        double* h = hist + d * bins + bin[d];
+        if (phases == 1) {
+            if (active) *h += value;
+        } else {
+            const int mine = phases == 2 ? interval & 1 : phases == 32 ? (int)(threadIdx.x & 31) : interval % phases;
+            for (int p = 0; p < phases; ++p) {
+                if (active && mine == p) *h += value;
+                __syncwarp();
+            }
         }
+        if (!counted && active) atomicAdd(&count[d * bins + bin[d]], 1);
     }
-    if (active) atomicAdd(&count[bin], 1);
+}
+
+// The counts of a warp's whole blocks (32 bins: one per lane), before the barrier.
+template <int D>
+__device__ __forceinline__ void add_whole_blocks(int whole, int32_t* count)
+{
+    if (whole > 0)
+        for (int d = 0; d < D; ++d) atomicAdd(&count[32 * d + (threadIdx.x & 31)], whole);
 }
 
 }  // namespace vegas
