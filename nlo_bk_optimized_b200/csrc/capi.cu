@@ -110,14 +110,22 @@ RhsBuffers carve(void* ws, int points)
 
 // A side stream for K1: K1 and K2+Kf read the same spline and active list and write
 // different buffers, so K1 runs beside K2+Kf and its last, partly filled wave of CTAs
-// overlaps the start of K2+Kf instead of idling most SMs.  One per evolve/rhs call.
+// overlaps the start of K2+Kf instead of idling most SMs.  Where K1 is the longer of the two it
+// goes first (a higher priority): K2+Kf CTAs that start ahead of it take slots that K1's clusters
+// of four then wait for (200 points, 2^14 samples, RK4 step: 545 us without, 470 with); a longer
+// K2+Kf keeps the default (400 points, 2^20 samples: 2 % slower with K1 ahead).  One per
+// evolve/rhs call.
 struct SideStream {
     cudaStream_t aux = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
     bool ok = false;
-    SideStream()
+    // A K1 evaluation costs about 2.6 K2+Kf evaluations, and a parent takes 192 (points - 1) of them.
+    static bool k1_longer(int points, double samples) { return samples < 500.0 * points; }
+    explicit SideStream(bool k1_first)
     {
-        ok = cudaStreamCreateWithFlags(&aux, cudaStreamNonBlocking) == cudaSuccess &&
+        int least = 0, greatest = 0;
+        cudaDeviceGetStreamPriorityRange(&least, &greatest);
+        ok = cudaStreamCreateWithPriority(&aux, cudaStreamNonBlocking, k1_first ? greatest : least) == cudaSuccess &&
              cudaEventCreateWithFlags(&fork, cudaEventDisableTiming) == cudaSuccess &&
              cudaEventCreateWithFlags(&join, cudaEventDisableTiming) == cudaSuccess;
         if (!ok) cudaGetLastError();  // fall back to one stream
@@ -187,6 +195,14 @@ struct StepGraph {
 // with 192-lane CTAs, not measured) launch every step.
 inline bool replay_pays(int points) { return points > 192; }
 
+// What turns the K2+Kf sums of a right-hand side into the integral (the Vegas values are integrals
+// already).
+double k2kf_factor(const nlo_bk_params& p, uint64_t samples, bool vegas)
+{
+    if (!order_has_nlo(p.order)) return 0.0;
+    return vegas ? 1.0 : samples ? 1.0 / (double)samples : 0.0;
+}
+
 int run_rhs(const nlo_bk_params& p, const double* r, const double* N, int points, const SobolDirsArg& dirs,
             uint64_t samples, const nlo_bk_box& box, double* dndy, double* k1_out, double* k2kf_out,
             const RhsBuffers& b, bool factor_ready, cudaStream_t stream, int shard = 0, int shards = 1,
@@ -203,17 +219,19 @@ int run_rhs(const nlo_bk_params& p, const double* r, const double* N, int points
         history.rows = rows;
         history.on = true;
     }
-    if ((e = launch_splines(r, single_row(N), points, 1, p.force_positive, b.factor, factor_ready ? 0 : 1, b.spline,
-                            stream)) !=
-        cudaSuccess)
-        return cuda_fail(e, "splines");
     // Sobol QMC: K2+Kf takes every active parent (a shard owns a range of Sobol indices), K1
     // the active parents i with i % shards == shard.  Vegas: both take the shard's parents.
     const bool split_samples = vegas == nullptr;
-    if ((e = launch_active(single_row(N), points, 1, split_samples ? 0 : shard, split_samples ? 1 : shards, b.active,
-                           b.count,
-                           stream)) != cudaSuccess)
-        return cuda_fail(e, "active");
+    RhsStart start;
+    start.active = b.active;
+    start.count = b.count;
+    start.shard = split_samples ? 0 : shard;
+    start.shards = split_samples ? 1 : shards;
+    start.k1 = b.k1;
+    start.k2kf = b.k2kf;
+    if ((e = launch_splines(r, single_row(N), points, 1, p.force_positive, b.factor, factor_ready ? 0 : 1, b.spline,
+                            stream, start)) != cudaSuccess)
+        return cuda_fail(e, "splines");
     const int32_t* k1_active = b.active;
     const int32_t* k1_count = b.count;
     if (shards > 1 && split_samples) {
@@ -230,21 +248,16 @@ int run_rhs(const nlo_bk_params& p, const double* r, const double* N, int points
         if ((e = cudaStreamWaitEvent(side->aux, side->fork, 0)) != cudaSuccess) return cuda_fail(e, "fork");
         k1_stream = side->aux;
     }
-    if ((e = launch_k1(p, r, points, b.spline, k1_active, k1_count, b.k1, k1_stream, history)) != cudaSuccess)
+    if ((e = launch_k1(p, r, points, b.spline, k1_active, k1_count, b.k1, k1_stream, history, 1, true)) != cudaSuccess)
         return cuda_fail(e, "k1");
     if (beside && (e = cudaEventRecord(side->join, side->aux)) != cudaSuccess) return cuda_fail(e, "join");
     // orders without NLO kernels (Order.has_nlo_kernels, bk/config.py:44-50) take no K2 + Kf:
-    // zero samples clear the sums and launch nothing
-    double k2kf_factor = 0.0;
+    // the sums stay cleared
     if (vegas) {
-        if (order_has_nlo(p.order)) {
-            if ((e = launch_k2kf_vegas(p, r, N, points, b.spline, shard, shards, dirs, box, *vegas, b.k2kf, stream)) !=
+        if (order_has_nlo(p.order) &&
+            (e = launch_k2kf_vegas(p, r, N, points, b.spline, shard, shards, dirs, box, *vegas, b.k2kf, stream)) !=
                 cudaSuccess)
-                return cuda_fail(e, "k2kf vegas");
-            k2kf_factor = 1.0;  // the Vegas values are integrals already
-        } else if ((e = cudaMemsetAsync(b.k2kf, 0, sizeof(double) * 3 * (size_t)points, stream)) != cudaSuccess) {
-            return cuda_fail(e, "k2kf clear");
-        }
+            return cuda_fail(e, "k2kf vegas");
     } else {
         const uint64_t nlo_samples = order_has_nlo(p.order) ? samples : 0;
         // this shard's Sobol indices [first, last) of the nlo_samples points; the sums are
@@ -252,16 +265,17 @@ int run_rhs(const nlo_bk_params& p, const double* r, const double* N, int points
         const uint64_t first = nlo_samples * (uint64_t)shard / (uint64_t)shards;
         const uint64_t last = nlo_samples * (uint64_t)(shard + 1) / (uint64_t)shards;
         if ((e = launch_k2kf(p, r, points, b.spline, b.active, b.count, dirs, first, last - first, box, b.k2kf,
-                             b.partial, b.k2kf_blocks, stream)) != cudaSuccess)
+                             b.partial, b.k2kf_blocks, stream, true)) != cudaSuccess)
             return cuda_fail(e, "k2kf");
-        k2kf_factor = nlo_samples ? 1.0 / (double)nlo_samples : 0.0;
     }
     if (beside && (e = cudaStreamWaitEvent(stream, side->join, 0)) != cudaSuccess) return cuda_fail(e, "join");
     // the replica refinement reads this right-hand side's K1
     if (vegas && order_has_nlo(p.order) && vegas->options.replicas > 0 &&
         (e = launch_k2kf_vegas_refine(p, r, N, points, b.spline, box, *vegas, b.k1, b.k2kf, stream)) != cudaSuccess)
         return cuda_fail(e, "k2kf vegas replicas");
-    if ((e = launch_assemble(b.k1, b.k2kf, points, k2kf_factor, dndy, k2kf_out, stream)) != cudaSuccess)
+    // dndy NULL: the caller assembles (launch_finish_stage)
+    if (dndy && (e = launch_assemble(b.k1, b.k2kf, points, k2kf_factor(p, samples, vegas != nullptr), dndy, k2kf_out,
+                                     stream)) != cudaSuccess)
         return cuda_fail(e, "assemble");
     if (k1_out) {
         if ((e = cudaMemcpyAsync(k1_out, b.k1, sizeof(double) * points, cudaMemcpyDeviceToDevice, stream)) !=
@@ -518,7 +532,7 @@ int nlo_bk_rhs(const nlo_bk_params* params, const double* r, const double* N, in
     if (!workspace || workspace_bytes < nlo_bk_rhs_workspace_bytes(points))
         return fail(NLO_ERR_WORKSPACE, "workspace too small for nlo_bk_rhs");
     const RhsBuffers b = carve(workspace, points);
-    const SideStream side;
+    const SideStream side(SideStream::k1_longer(points, (double)samples));
     return run_rhs(*params, r, N, points, to_arg(dirs), (uint64_t)samples, *box, dndy, k1, k2kf, b, false,
                    (cudaStream_t)stream, 0, 1, nullptr, nullptr, 0, &side);
 }
@@ -540,7 +554,7 @@ int nlo_bk_rhs_shard(const nlo_bk_params* params, const double* r, const double*
     if (!workspace || workspace_bytes < nlo_bk_rhs_workspace_bytes(points))
         return fail(NLO_ERR_WORKSPACE, "workspace too small for nlo_bk_rhs_shard");
     const RhsBuffers b = carve(workspace, points);
-    const SideStream side;
+    const SideStream side(SideStream::k1_longer(points, (double)samples));
     return run_rhs(*params, r, N, points, to_arg(dirs), (uint64_t)samples, *box, dndy, nullptr, nullptr, b, false,
                    (cudaStream_t)stream, shard, shards, nullptr, nullptr, 0, &side);
 }
@@ -573,7 +587,7 @@ int nlo_bk_rhs_history(const nlo_bk_params* params, const double* r, int32_t poi
         return fail(NLO_ERR_WORKSPACE, "workspace too small for nlo_bk_rhs_history");
     const RhsBuffers b = carve(workspace, points);
     const double* N = hist_N + (size_t)(rows - 1) * points;
-    const SideStream side;
+    const SideStream side(SideStream::k1_longer(points, (double)samples));
     return run_rhs(*params, r, N, points, to_arg(dirs), (uint64_t)samples, *box, dndy, k1, k2kf, b, false,
                    (cudaStream_t)stream, 0, 1, hist_y, hist_N, rows, &side);
 }
@@ -611,7 +625,7 @@ static int evolve_rows(const nlo_bk_params* params, const double* r, int32_t poi
     cudaError_t e = cudaMemsetAsync(status, 0, sizeof(uint32_t), s);
     if (e != cudaSuccess) return cuda_fail(e, "status reset");
     const int clamp = params->force_positive ? 1 : 0;
-    const SideStream side;
+    const SideStream side(!vegas && SideStream::k1_longer(points, (double)samples));
     // the spline factorisation depends on the grid only: form it on the first stage
     bool factor_ready = false;
     // the steps of a fixed-step Sobol evolution are all alike: after the first (launched one
@@ -621,18 +635,21 @@ static int evolve_rows(const nlo_bk_params* params, const double* r, int32_t poi
     const bool replay = !params->kinematical_constraint && !vegas && steps > 1 && replay_pays(points);
     StepGraph graph;
     bool recorded = false;
+    const double factor = k2kf_factor(*params, (uint64_t)samples, vegas != nullptr);
     auto step_from = [&](const double* N, double* next, int it, cudaStream_t st) {
+        int latest = 0;  // the derivative that the stage's combination assembles
         auto rhs = [&](int src, int k) {
-            const int code = run_rhs(*params, r, src < 0 ? N : tmp, points, dirs_arg, (uint64_t)samples, *box, kk[k],
+            const int code = run_rhs(*params, r, src < 0 ? N : tmp, points, dirs_arg, (uint64_t)samples, *box, nullptr,
                                      nullptr, nullptr, b, factor_ready, st, 0, 1, y, table, it + 1, &side, vegas);
+            latest = k;
             factor_ready = true;
             return code;
         };
         auto comb = [&](int nk, const int* ks, const double* coef, int dst) {
             const double* kp[4];
             for (int j = 0; j < nk; ++j) kp[j] = kk[ks[j]];
-            const cudaError_t err = launch_axpy_stage(N, kp, coef, nk, points, dst ? next : tmp, dst ? clamp : 0,
-                                                      dst ? status : nullptr, st);
+            const cudaError_t err = launch_finish_stage(b.k1, b.k2kf, factor, kk[latest], N, kp, coef, nk, points,
+                                                        dst ? next : tmp, dst ? clamp : 0, dst ? status : nullptr, st);
             return err == cudaSuccess ? NLO_OK : cuda_fail(err, "stage");
         };
         return step_sequence(stepper, step, rhs, comb);
@@ -772,7 +789,7 @@ int nlo_bk_rhs_vegas(const nlo_bk_params* params, const double* r, int32_t point
     std::vector<SobolDirsArg> replica_dirs;
     const BkVegasCall call = vegas_call(workspace, points, options, state, dirs, replica_dirs);
     const double* N = hist_N + (size_t)(rows - 1) * points;
-    const SideStream side;
+    const SideStream side(false);
     return run_rhs(*params, r, N, points, to_arg(dirs), (uint64_t)options->samples_per_iteration, *box, dndy, k1, k2kf,
                    b, false, (cudaStream_t)stream, shard, shards, hist_y, hist_N, rows, &side, &call);
 }
@@ -872,47 +889,49 @@ int nlo_bk_evolve_sets(const nlo_bk_params* params, const double* r, int32_t poi
     fixed.base = cur;
     fixed.stride = n;
     const int clamp = params->force_positive ? 1 : 0;
-    const SideStream side;
+    double mean_samples = 0.0;
+    for (int i = 0; i < sets; ++i) mean_samples += (double)samples[i] / sets;
+    const SideStream side(SideStream::k1_longer(points, mean_samples));
     bool factor_ready = false;
     // as in evolve_rows: the first step launches its kernels one by one, the later ones
     // replay a recording of one step that advances the fixed rows in place
     StepGraph graph;
     bool recorded = false;
     auto step_from = [&](const RowsArg& now, const RowsArg& next, cudaStream_t s) {
+        int latest = 0;  // the derivative that the stage's combination assembles
         auto rhs = [&](int src, int k) {
             const RowsArg& in = src < 0 ? now : work;
+            RhsStart start;
+            start.active = active;
+            start.count = counts;
+            start.k1 = k1;
+            start.k2kf = k2kf;
             if ((e = launch_splines(r, in, points, sets, params->force_positive, factor, factor_ready ? 0 : 1, spline,
-                                    s)) != cudaSuccess)
+                                    s, start)) != cudaSuccess)
                 return cuda_fail(e, "splines");
             factor_ready = true;
-            if ((e = launch_active(in, points, sets, 0, 1, active, counts, s)) != cudaSuccess)
-                return cuda_fail(e, "active");
+            latest = k;
             const bool beside = side.ok;
             cudaStream_t k1_stream = beside ? side.aux : s;
             if (beside && ((e = cudaEventRecord(side.fork, s)) != cudaSuccess ||
                            (e = cudaStreamWaitEvent(side.aux, side.fork, 0)) != cudaSuccess))
                 return cuda_fail(e, "fork");
-            if ((e = launch_k1(*params, r, points, spline, active, counts, k1, k1_stream, K1History(), sets)) !=
+            if ((e = launch_k1(*params, r, points, spline, active, counts, k1, k1_stream, K1History(), sets, true)) !=
                 cudaSuccess)
                 return cuda_fail(e, "k1");
             if (beside && (e = cudaEventRecord(side.join, side.aux)) != cudaSuccess) return cuda_fail(e, "join");
-            if (nlo) {
-                if ((e = launch_k2kf_sets(*params, r, points, sets, spline, spline_doubles(points), active, counts,
-                                          *box, L, table, k2kf, partial, s)) != cudaSuccess)
-                    return cuda_fail(e, "k2kf sets");
-            } else if ((e = cudaMemsetAsync(k2kf, 0, sizeof(double) * 3 * S * n, s)) != cudaSuccess) {
-                return cuda_fail(e, "k2kf clear");
-            }
+            if (nlo && (e = launch_k2kf_sets(*params, r, points, sets, spline, spline_doubles(points), active, counts,
+                                             *box, L, table, k2kf, partial, s, true)) != cudaSuccess)
+                return cuda_fail(e, "k2kf sets");
             if (beside && (e = cudaStreamWaitEvent(s, side.join, 0)) != cudaSuccess) return cuda_fail(e, "join");
-            if ((e = launch_assemble_sets(k1, k2kf, points, sets, table, kk[k], s)) != cudaSuccess)
-                return cuda_fail(e, "assemble");
             return (int)NLO_OK;
         };
         auto comb = [&](int nk, const int* ks, const double* coef, int dst) {
             const double* kp[4];
             for (int j = 0; j < nk; ++j) kp[j] = kk[ks[j]];
-            const cudaError_t err = launch_axpy_sets(now, kp, coef, nk, points, sets, dst ? next : work,
-                                                     dst ? clamp : 0, dst ? status : nullptr, s);
+            const cudaError_t err = launch_finish_stage_sets(k1, k2kf, table, kk[latest], now, kp, coef, nk, points,
+                                                             sets, dst ? next : work, dst ? clamp : 0,
+                                                             dst ? status : nullptr, s);
             return err == cudaSuccess ? (int)NLO_OK : cuda_fail(err, "stage");
         };
         return step_sequence(stepper, step, rhs, comb);

@@ -15,15 +15,21 @@ namespace nlo {
 
 namespace {
 
+// dN/dY of one parent: K1 + (K2 + Kf), 0 where it is not finite.
+__device__ __forceinline__ double assembled(double k1, const double* __restrict__ sums, double factor, double& nlo)
+{
+    nlo = (sums[0] + sums[1]) * factor;
+    const double v = k1 + nlo;
+    return isfinite(v) ? v : 0.0;
+}
+
 __global__ void assemble_kernel(const double* __restrict__ k1, const double* __restrict__ k2kf, int n,
                                 double inv_samples, double* __restrict__ dndy, double* __restrict__ k2kf_total)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    const double nlo = (k2kf[3 * i] + k2kf[3 * i + 1]) * inv_samples;
-    double v = k1[i] + nlo;
-    if (!isfinite(v)) v = 0.0;
-    dndy[i] = v;
+    double nlo;
+    dndy[i] = assembled(k1[i], k2kf + 3 * (size_t)i, inv_samples, nlo);
     if (k2kf_total) k2kf_total[i] = nlo;
 }
 
@@ -33,30 +39,47 @@ struct StageArgs {
     int nk;
 };
 
-__global__ void axpy_stage_kernel(const double* __restrict__ N, StageArgs a, int n, double* __restrict__ out,
-                                  int clamp, uint32_t* __restrict__ status)
+__device__ __forceinline__ double combined(double v, const StageArgs& a, size_t at, int clamp, uint32_t* status)
+{
+    for (int j = 0; j < a.nk; ++j) v += a.c[j] * a.k[j][at];
+    if (clamp) v = v < 0.0 ? 0.0 : (v > 1.0 ? 1.0 : v);
+    if (status && !isfinite(v)) atomicOr(status, (uint32_t)kStatusNonFinite);
+    return v;
+}
+
+__global__ void axpy_stage_kernel(const double* N, StageArgs a, int n, double* out, int clamp,
+                                  uint32_t* __restrict__ status)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double v = N[i];
-    for (int j = 0; j < a.nk; ++j) v += a.c[j] * a.k[j][i];
-    if (clamp) v = v < 0.0 ? 0.0 : (v > 1.0 ? 1.0 : v);
-    if (status && !isfinite(v)) atomicOr(status, (uint32_t)kStatusNonFinite);
-    out[i] = v;
+    out[i] = combined(N[i], a, i, clamp, status);
+}
+
+// The end of a stage in one launch: the derivative of each parent, then the stage combination,
+// whose terms read this thread's element only (the last of them just written).
+__global__ void finish_stage_kernel(const double* __restrict__ k1, const double* __restrict__ k2kf, double factor,
+                                    double* dndy, const double* N, StageArgs a, int n, double* out, int clamp,
+                                    uint32_t* __restrict__ status)
+{
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    double nlo;
+    dndy[i] = assembled(k1[i], k2kf + 3 * (size_t)i, factor, nlo);
+    out[i] = combined(N[i], a, i, clamp, status);
 }
 
 // Several parameter sets: blockIdx.y is the set.
-__global__ void assemble_sets_kernel(const double* __restrict__ k1, const double* __restrict__ k2kf, int n,
-                                     const SetTable* __restrict__ table, double* __restrict__ dndy)
+__global__ void finish_stage_sets_kernel(const double* __restrict__ k1, const double* __restrict__ k2kf,
+                                         const SetTable* __restrict__ table, double* dndy, RowsArg N, StageArgs a,
+                                         int n, RowsArg out, int clamp, uint32_t* __restrict__ status)
 {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = blockIdx.y;
     if (i >= n) return;
-    const double* q = k2kf + 3 * ((size_t)s * n + i);
-    const double nlo = (q[0] + q[1]) * table->inv[s];
-    double v = k1[(size_t)s * n + i] + nlo;
-    if (!isfinite(v)) v = 0.0;
-    dndy[(size_t)s * n + i] = v;
+    const size_t at = (size_t)s * n + i;
+    double nlo;
+    dndy[at] = assembled(k1[at], k2kf + 3 * at, table->inv[s], nlo);
+    out.at(s)[i] = combined(N.at(s)[i], a, at, clamp, status ? status + s : nullptr);
 }
 
 __global__ void axpy_sets_kernel(RowsArg N, StageArgs a, int n, RowsArg out, int clamp, uint32_t* __restrict__ status)
@@ -64,11 +87,7 @@ __global__ void axpy_sets_kernel(RowsArg N, StageArgs a, int n, RowsArg out, int
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     const int s = blockIdx.y;
     if (i >= n) return;
-    double v = N.at(s)[i];
-    for (int j = 0; j < a.nk; ++j) v += a.c[j] * a.k[j][(size_t)s * n + i];
-    if (clamp) v = v < 0.0 ? 0.0 : (v > 1.0 ? 1.0 : v);
-    if (status && !isfinite(v)) atomicOr(status + s, (uint32_t)kStatusNonFinite);
-    out.at(s)[i] = v;
+    out.at(s)[i] = combined(N.at(s)[i], a, (size_t)s * n + i, clamp, status ? status + s : nullptr);
 }
 
 struct SetupArg {
@@ -141,15 +160,7 @@ cudaError_t launch_sets_setup(double* const* rows, const int64_t* samples, const
     return e;
 }
 
-cudaError_t launch_assemble_sets(const double* k1, const double* k2kf, int points, int sets, const SetTable* table,
-                                 double* dndy, cudaStream_t stream)
-{
-    assemble_sets_kernel<<<dim3((points + 255) / 256, sets), 256, 0, stream>>>(k1, k2kf, points, table, dndy);
-    return cudaGetLastError();
-}
-
-cudaError_t launch_axpy_sets(const RowsArg& N, const double* const* k, const double* coef, int nk, int points,
-                             int sets, const RowsArg& out, int clamp, uint32_t* status, cudaStream_t stream)
+static StageArgs stage_args(const double* const* k, const double* coef, int nk)
 {
     StageArgs a;
     a.nk = nk;
@@ -157,7 +168,32 @@ cudaError_t launch_axpy_sets(const RowsArg& N, const double* const* k, const dou
         a.k[j] = j < nk ? k[j] : nullptr;
         a.c[j] = j < nk ? coef[j] : 0.0;
     }
-    axpy_sets_kernel<<<dim3((points + 255) / 256, sets), 256, 0, stream>>>(N, a, points, out, clamp, status);
+    return a;
+}
+
+cudaError_t launch_finish_stage(const double* k1, const double* k2kf, double factor, double* dndy, const double* N,
+                                const double* const* k, const double* coef, int nk, int points, double* out,
+                                int clamp, uint32_t* status, cudaStream_t stream)
+{
+    finish_stage_kernel<<<(points + 127) / 128, 128, 0, stream>>>(k1, k2kf, factor, dndy, N, stage_args(k, coef, nk),
+                                                                  points, out, clamp, status);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_finish_stage_sets(const double* k1, const double* k2kf, const SetTable* table, double* dndy,
+                                     const RowsArg& N, const double* const* k, const double* coef, int nk, int points,
+                                     int sets, const RowsArg& out, int clamp, uint32_t* status, cudaStream_t stream)
+{
+    finish_stage_sets_kernel<<<dim3((points + 255) / 256, sets), 256, 0, stream>>>(
+        k1, k2kf, table, dndy, N, stage_args(k, coef, nk), points, out, clamp, status);
+    return cudaGetLastError();
+}
+
+cudaError_t launch_axpy_sets(const RowsArg& N, const double* const* k, const double* coef, int nk, int points,
+                             int sets, const RowsArg& out, int clamp, uint32_t* status, cudaStream_t stream)
+{
+    axpy_sets_kernel<<<dim3((points + 255) / 256, sets), 256, 0, stream>>>(N, stage_args(k, coef, nk), points, out,
+                                                                           clamp, status);
     return cudaGetLastError();
 }
 
@@ -171,13 +207,8 @@ cudaError_t launch_assemble(const double* k1, const double* k2kf, int points, do
 cudaError_t launch_axpy_stage(const double* N, const double* const* k, const double* coef, int nk, int points,
                               double* out, int clamp, uint32_t* status, cudaStream_t stream)
 {
-    StageArgs a;
-    a.nk = nk;
-    for (int j = 0; j < 4; ++j) {
-        a.k[j] = j < nk ? k[j] : nullptr;
-        a.c[j] = j < nk ? coef[j] : 0.0;
-    }
-    axpy_stage_kernel<<<(points + 255) / 256, 256, 0, stream>>>(N, a, points, out, clamp, status);
+    axpy_stage_kernel<<<(points + 255) / 256, 256, 0, stream>>>(N, stage_args(k, coef, nk), points, out, clamp,
+                                                                status);
     return cudaGetLastError();
 }
 

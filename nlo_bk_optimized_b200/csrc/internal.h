@@ -97,7 +97,7 @@ cudaError_t launch_sets_setup(double* const* rows, const int64_t* samples, const
 cudaError_t launch_k2kf_sets(const nlo_bk_params& p, const double* r, int points, int sets, const double* spline,
                              size_t spline_stride, const int32_t* active, const int32_t* counts,
                              const nlo_bk_box& box, const SetsLayout& L, const SetTable* table, double* out,
-                             double* partial, cudaStream_t stream);
+                             double* partial, cudaStream_t stream, bool cleared = false);
 
 // Records a message for nlo_last_error() and returns code.
 int set_last_error(int code, const char* message);
@@ -109,10 +109,21 @@ cudaError_t raise_dynamic_smem(const void* func, size_t bytes);
 // L1: ask for the largest shared-memory carveout, once per kernel and device.
 cudaError_t prefer_shared_carveout(const void* func);
 
+// What a right-hand side begins with besides the refit (NULL: left out): the active parents of
+// each row (index % shards == shard; active + s * n, count + s) and the cleared K1 (+ s * n) and
+// K2+Kf sums (+ s * 3n).
+struct RhsStart {
+    int32_t* active = nullptr;
+    int32_t* count = nullptr;
+    int shard = 0, shards = 1;
+    double* k1 = nullptr;
+    double* k2kf = nullptr;
+};
 // Spline tables of `sets` rows: set s reads N.at(s) and writes out + s * spline_doubles(n)
 // and its factorisation at factor + s * 2n.
 cudaError_t launch_splines(const double* r, const RowsArg& N, int n, int sets, int force_positive, double* factor,
-                           int compute_factor, double* out, cudaStream_t stream);
+                           int compute_factor, double* out, cudaStream_t stream,
+                           const RhsStart& start = RhsStart());
 // active parents (index > 0, N <= 0.99999) with index % shards == shard; set s reads N.at(s)
 // and writes active + s * n and count + s
 cudaError_t launch_active(const RowsArg& N, int n, int sets, int shard, int shards, int32_t* active, int32_t* count,
@@ -133,15 +144,16 @@ constexpr int kKcStride = 14;  // per r interval: start, local interval, 2 x 6 w
 inline size_t kc_weights_doubles(int points) { return (size_t)(points - 1) * kKcStride; }
 cudaError_t launch_kc_weights(const double* r, int points, double* weights, cudaStream_t stream);
 
+// (`cleared`: the caller has cleared `out`.)
 // K1 of `sets` sets: set s reads spline + s * spline_doubles(points), active + s * points and
 // count + s, and writes out + s * points (the constraint history: one set only).
 cudaError_t launch_k1(const nlo_bk_params& p, const double* r, int points, const double* spline,
                       const int32_t* active, const int32_t* count, double* out, cudaStream_t stream,
-                      const K1History& history = K1History(), int sets = 1);
+                      const K1History& history = K1History(), int sets = 1, bool cleared = false);
 cudaError_t launch_k2kf(const nlo_bk_params& p, const double* r, int points, const double* spline,
                         const int32_t* active, const int32_t* count, const SobolDirsArg& dirs, uint64_t offset,
                         uint64_t samples, const nlo_bk_box& box, double* out, double* partial, int max_blocks,
-                        cudaStream_t stream);
+                        cudaStream_t stream, bool cleared = false);
 // K2+Kf by Vegas (k2kf_vegas.cu): the per-call buffers, carved from the caller's workspace.
 struct BkVegasCall {
     nlo_bk_vegas_options options;
@@ -174,11 +186,17 @@ cudaError_t vegas_launch_reduce(const double* partial, int keys, int blocks_per_
 
 cudaError_t launch_assemble(const double* k1, const double* k2kf, int points, double inv_samples, double* dndy,
                             double* k2kf_total, cudaStream_t stream);
+// launch_assemble into dndy, then launch_axpy_stage whose last term k[nk - 1] is dndy.
+cudaError_t launch_finish_stage(const double* k1, const double* k2kf, double factor, double* dndy, const double* N,
+                                const double* const* k, const double* coef, int nk, int points, double* out,
+                                int clamp, uint32_t* status, cudaStream_t stream);
 cudaError_t launch_axpy_stage(const double* N, const double* const* k, const double* coef, int nk, int points,
                               double* out, int clamp, uint32_t* status, cudaStream_t stream);
-// Several sets: dndy + s * points = k1 + s * points + (k2kf + s * 3 points) * table->inv[s].
-cudaError_t launch_assemble_sets(const double* k1, const double* k2kf, int points, int sets, const SetTable* table,
-                                 double* dndy, cudaStream_t stream);
+// Several sets: dndy + s * points = k1 + s * points + (k2kf + s * 3 points) * table->inv[s], then
+// launch_axpy_sets whose last term is dndy.
+cudaError_t launch_finish_stage_sets(const double* k1, const double* k2kf, const SetTable* table, double* dndy,
+                                     const RowsArg& N, const double* const* k, const double* coef, int nk, int points,
+                                     int sets, const RowsArg& out, int clamp, uint32_t* status, cudaStream_t stream);
 // Several sets: out.at(s) = N.at(s) + sum_j coef[j] (k[j] + s * points); status + s when given.
 cudaError_t launch_axpy_sets(const RowsArg& N, const double* const* k, const double* coef, int nk, int points,
                              int sets, const RowsArg& out, int clamp, uint32_t* status, cudaStream_t stream);

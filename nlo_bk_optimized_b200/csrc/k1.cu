@@ -804,7 +804,7 @@ cudaError_t launch_kc_weights(const double* r, int points, double* weights, cuda
 
 cudaError_t launch_k1(const nlo_bk_params& p, const double* r, int points, const double* spline,
                       const int32_t* active, const int32_t* count, double* out, cudaStream_t stream,
-                      const K1History& history, int sets)
+                      const K1History& history, int sets, bool cleared)
 {
     if (history.on && sets != 1) return cudaErrorInvalidValue;
     K1Consts consts;
@@ -816,7 +816,7 @@ cudaError_t launch_k1(const nlo_bk_params& p, const double* r, int points, const
         consts.sh2[j] = sh * sh;
         consts.aw[j] = consts.rule.w24[j] * kPi * v;
     }
-    cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double) * (size_t)points * sets, stream);
+    cudaError_t e = cleared ? cudaSuccess : cudaMemsetAsync(out, 0, sizeof(double) * (size_t)points * sets, stream);
     if (e != cudaSuccess) return e;
     const Phys<double> phd = make_phys<double>(p);
     const size_t per_split = (size_t)((points - 1 + kK1Split - 1) / kK1Split) * 8;

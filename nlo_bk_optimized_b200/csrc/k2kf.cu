@@ -62,7 +62,8 @@ __global__ void __launch_bounds__(448, (sizeof(T) == 4 ? 2 : 1)) k2kf_kernel(Phy
                                                     const double* __restrict__ spline,
                                                     const int32_t* __restrict__ active,
                                                     const int32_t* __restrict__ count, uint64_t offset,
-                                                    uint64_t samples, double* __restrict__ partial, SetsArg sa)
+                                                    uint64_t samples, int tile_samples, double* __restrict__ partial,
+                                                    SetsArg sa)
 {
     const int slots = MULTI ? sa.per_cta : 1;
     const int lanes = MULTI ? sa.lanes : (int)blockDim.x;
@@ -78,7 +79,7 @@ __global__ void __launch_bounds__(448, (sizeof(T) == 4 ? 2 : 1)) k2kf_kernel(Phy
         // slot 0 of a group holds its largest budget
         max_samples = sa.table->samples[sa.table->slot_set[group * slots]];
     }
-    const uint64_t tile = lanes;
+    const uint64_t tile = MULTI ? lanes : tile_samples;
     const uint64_t tiles = (max_samples + tile - 1) / tile;
     // MULTI: a CTA past its group's tiles has nothing to add (the finalize reads only the CTAs
     // below the tile count)
@@ -184,11 +185,13 @@ __global__ void __launch_bounds__(448, (sizeof(T) == 4 ? 2 : 1)) k2kf_kernel(Phy
                 // pair layout: the fields of samples 2p and 2p+1 side by side (lanes is even;
                 // a padding sample past the budget carries zero weight)
                 float rec[kRecLen];
-                k2_prepare<float>(s, box, my_st, my_st + 120, offset + local, local < my_samples, rec);
-                float* dst = reinterpret_cast<float*>(recs) + (size_t)(threadIdx.x >> 1) * (2 * kRecLen) +
-                             (threadIdx.x & 1);
+                if (lt < (int)tile) {
+                    k2_prepare<float>(s, box, my_st, my_st + 120, offset + local, local < my_samples, rec);
+                    float* dst = reinterpret_cast<float*>(recs) + (size_t)(threadIdx.x >> 1) * (2 * kRecLen) +
+                                 (threadIdx.x & 1);
 #pragma unroll
-                for (int f = 0; f < kRecLen; ++f) dst[2 * f] = rec[f];
+                    for (int f = 0; f < kRecLen; ++f) dst[2 * f] = rec[f];
+                }
                 __syncthreads();
                 if (has_parent) {
                     const float4* pr = reinterpret_cast<const float4*>(recs) + (rec0 / 2) * (kRecLen / 2);
@@ -215,7 +218,9 @@ __global__ void __launch_bounds__(448, (sizeof(T) == 4 ? 2 : 1)) k2kf_kernel(Phy
                     acc_sq += (double)sq.x + (double)sq.y;
                 }
             } else {
-                k2_prepare<T>(s, box, my_st, my_st + 120, offset + local, local < my_samples, recs[threadIdx.x].v);
+                if (lt < (int)tile)
+                    k2_prepare<T>(s, box, my_st, my_st + 120, offset + local, local < my_samples,
+                                  recs[threadIdx.x].v);
                 __syncthreads();
                 if (has_parent) {
                     Kahan<T> sk2, skf;
@@ -362,7 +367,8 @@ cudaError_t launch_sets_typed(const nlo_bk_params& p, const double* r, int point
     SobolDirsArg unused;
     std::memset(&unused, 0, sizeof(unused));
     k2kf_kernel<T, SYM, COUPLING, true><<<grid, L.threads, smem, stream>>>(
-        make_phys<T>(p), make_box<T>(p, box, SYM), unused, r, points, spline, active, counts, 0, 0, partial, sa);
+        make_phys<T>(p), make_box<T>(p, box, SYM), unused, r, points, spline, active, counts, 0, 0, L.lanes, partial,
+        sa);
     return cudaGetLastError();
 }
 
@@ -383,16 +389,30 @@ cudaError_t launch_typed(const nlo_bk_params& p, const double* r, int points, co
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (per_sm < 1) per_sm = 1;
-    const uint64_t tiles = (samples + threads - 1) / threads;
     uint64_t blocks = (uint64_t)per_sm * sms / (uint64_t)parent_tiles;
     if (blocks < 1) blocks = 1;
     if (blocks > (uint64_t)max_blocks) blocks = (uint64_t)max_blocks;
+    // The tile (a multiple of the 32 samples of an FP32 partial sum, at most one sample per thread)
+    // for which a CTA's share of the samples rounds up least, with 8 samples' worth of staging a
+    // tile: whole tiles of 416 gave 2^20 samples over 296 CTAs 8 tiles for some and 9 for others
+    // (3,744 samples' time; 14 tiles of 256 are 3,584), and 2^14 samples at 200 parents 74 CTAs
+    // with one tile of 224 each (512 of 32).
+    const uint64_t share = (samples + blocks - 1) / blocks;
+    uint64_t tile = (uint64_t)threads, best = ~(uint64_t)0;
+    for (uint64_t t = 32; t <= (uint64_t)threads; t += 32) {
+        const uint64_t cost = (share + t - 1) / t * (t + 8);
+        if (cost <= best) {
+            best = cost;
+            tile = t;
+        }
+    }
+    const uint64_t tiles = (samples + tile - 1) / tile;
     if (blocks > tiles) blocks = tiles;
     *used_blocks = (int)blocks;
     dim3 grid((unsigned)blocks, (unsigned)parent_tiles);
     k2kf_kernel<T, SYM, COUPLING, false><<<grid, threads, smem, stream>>>(
-        make_phys<T>(p), make_box<T>(p, box, SYM), dirs, r, points, spline, active, count, offset, samples, partial,
-        SetsArg{});
+        make_phys<T>(p), make_box<T>(p, box, SYM), dirs, r, points, spline, active, count, offset, samples, (int)tile,
+        partial, SetsArg{});
     return cudaGetLastError();
 }
 
@@ -405,9 +425,9 @@ constexpr int kLaneCap = 448;
 cudaError_t launch_k2kf(const nlo_bk_params& p, const double* r, int points, const double* spline,
                         const int32_t* active, const int32_t* count, const SobolDirsArg& dirs, uint64_t offset,
                         uint64_t samples, const nlo_bk_box& box, double* out, double* partial, int max_blocks,
-                        cudaStream_t stream)
+                        cudaStream_t stream, bool cleared)
 {
-    cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double) * 3 * (size_t)points, stream);
+    cudaError_t e = cleared ? cudaSuccess : cudaMemsetAsync(out, 0, sizeof(double) * 3 * (size_t)points, stream);
     if (e != cudaSuccess || samples == 0) return e;
     int threads = ((points < kLaneCap ? points : kLaneCap) + 31) / 32 * 32;
     if (threads < 64) threads = 64;
@@ -449,9 +469,9 @@ SetsLayout sets_layout(int points, int sets, int waves)
 cudaError_t launch_k2kf_sets(const nlo_bk_params& p, const double* r, int points, int sets, const double* spline,
                              size_t spline_stride, const int32_t* active, const int32_t* counts,
                              const nlo_bk_box& box, const SetsLayout& L, const SetTable* table, double* out,
-                             double* partial, cudaStream_t stream)
+                             double* partial, cudaStream_t stream, bool cleared)
 {
-    cudaError_t e = cudaMemsetAsync(out, 0, sizeof(double) * 3 * (size_t)points * sets, stream);
+    cudaError_t e = cleared ? cudaSuccess : cudaMemsetAsync(out, 0, sizeof(double) * 3 * (size_t)points * sets, stream);
     if (e != cudaSuccess) return e;
     e = dispatch_variant(p, [&](auto t, auto sym, auto c) {
         return launch_sets_typed<decltype(t), decltype(sym)::value, decltype(c)::value>(

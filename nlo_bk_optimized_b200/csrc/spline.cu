@@ -5,8 +5,8 @@
 // Thomas solve, log-log table with -40 for non-positive values) for the two
 // evolution rows of bk/evolution.py:548-560: log N with N clamped to [0,1], and
 // log S with S = 1 - N clamped to [0,1], evaluated as log1p(-N) so that S close to
-// 1 keeps the relative precision of N.  One CTA per row pair; the two Thomas
-// sweeps run concurrently in two warps.
+// 1 keeps the relative precision of N.  One CTA per row pair; the two rows' Thomas
+// sweeps run concurrently in two warps, as scans over the warp.
 
 #include <cuda_runtime.h>
 
@@ -16,115 +16,45 @@
 
 namespace nlo {
 
-// factor: [2][n] = 1/denominator and upper coefficient of the Thomas sweep for
-// the natural-spline system on the knots log r (it depends on the grid only).
-// With compute_factor set, thread 0 forms it first (and stores it for later calls).
-// One CTA per set (blockIdx.x): row N.at(set), tables at out + set * spline_doubles(n), its own
-// factorisation copy at factor + set * 2n.
-__global__ void __launch_bounds__(256) splines_kernel(const double* __restrict__ r, RowsArg rows,
-                                                      int n, int force_positive, double* __restrict__ factor,
-                                                      int compute_factor, double* __restrict__ out)
+// s_i = c_i + a_i s_{i-1} over i = 0..m-1 (REVERSE: s_i = c_i + a_i s_{i+1} from the other end), in
+// place over c, by one warp: a lane composes the affine maps of its consecutive elements, a
+// warp scan composes the lanes', and each lane walks its elements again from its carry-in.
+// m = 398: 13 elements twice and 5 scan steps instead of a chain of 398.
+template <bool REVERSE>
+__device__ __forceinline__ void warp_affine_scan(const double* a, double* c, int m)
 {
-    const double* __restrict__ N = rows.at(blockIdx.x);
-    factor += (size_t)blockIdx.x * 2 * n;
-    out += (size_t)blockIdx.x * spline_doubles(n);
-    extern __shared__ double smem[];
-    double* x = smem;             // [n]
-    double* y = x + n;            // [2][n]
-    double* rhs = y + 2 * n;      // [2][n]
-    double* sol = rhs + 2 * n;    // [2][n]
-    double* inv_den = sol + 2 * n;  // [n]
-    double* up = inv_den + n;       // [n]
-    const int m = n - 2;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        x[i] = log(r[i]);
-        out[i] = x[i];
-        const double v = N[i];
-        // log N row: N > 1 -> 1; force_positive: N < 0 -> 0
-        double vn = v > 1.0 ? 1.0 : v;
-        if (force_positive && vn < 0.0) vn = 0.0;
-        y[i] = vn > 0.0 ? log(vn) : kMinLog;
-        // log S row: S = 1 - N; S < 0 -> 0; force_positive: S > 1 -> 1
-        double ns = v;
-        if (force_positive && ns < 0.0) ns = 0.0;
-        y[n + i] = ns < 1.0 ? log1p(-ns) : kMinLog;
+    const int lane = threadIdx.x & 31;
+    const int per = (m + 31) / 32;
+    const int begin = min(lane * per, m), end = min(begin + per, m);
+    auto at = [&](int i) { return REVERSE ? m - 1 - i : i; };
+    double A = 1.0, C = 0.0;
+    for (int i = begin; i < end; ++i) {
+        const int k = at(i);
+        C = fma(a[k], C, c[k]);
+        A *= a[k];
     }
-    __syncthreads();
-    for (int item = threadIdx.x; item < 2 * m; item += blockDim.x) {
-        const int row = item / m, i = item - row * m;
-        const double* yy = y + row * n;
-        rhs[row * n + i] =
-            6.0 * ((yy[i + 2] - yy[i + 1]) / (x[i + 2] - x[i + 1]) - (yy[i + 1] - yy[i]) / (x[i + 1] - x[i]));
-    }
-    if (compute_factor && threadIdx.x == 0 && m >= 1) {
-        // denominators of the forward sweep (interpolation.py:124-149)
-        double d = 2.0 * ((x[1] - x[0]) + (x[2] - x[1]));
-        factor[0] = 1.0 / d;
-        for (int i = 1; i < m; ++i) {
-            const double upper_prev = (x[i + 1] - x[i]) * factor[i - 1];
-            factor[n + i - 1] = upper_prev;
-            d = 2.0 * ((x[i + 1] - x[i]) + (x[i + 2] - x[i + 1])) - (x[i + 1] - x[i]) * upper_prev;
-            factor[i] = 1.0 / d;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const double A1 = __shfl_up_sync(0xffffffffu, A, o), C1 = __shfl_up_sync(0xffffffffu, C, o);
+        if (lane >= o) {
+            C = fma(A, C1, C);
+            A *= A1;
         }
     }
-    __syncthreads();
-    // The forward sweep s_i = (b_i - h_i s_{i-1}) / d_i as s_i = c_i + a_i s_{i-1} with
-    // c_i = b_i / d_i and a_i = -h_i / d_i formed in parallel, so the sequential chain is
-    // one FMA a step whose operands load ahead of it; the back substitution likewise
-    // with the negated upper diagonal.
-    for (int item = threadIdx.x; item < 2 * m; item += blockDim.x) {
-        const int row = item / m, i = item - row * m;
-        rhs[row * n + i] *= factor[i];
-        if (row == 0) {
-            inv_den[i] = i > 0 ? -(x[i + 1] - x[i]) * factor[i] : 0.0;
-            up[i] = i < m - 1 ? -factor[n + i] : 0.0;
-        }
-    }
-    __syncthreads();
-    // warp 0 solves row 0, warp 1 row 1
-    if ((threadIdx.x & 31) == 0 && threadIdx.x < 64 && m >= 1) {
-        const int row = threadIdx.x >> 5;
-        const double* c = rhs + row * n;
-        double* s = sol + row * n;
-        double prev = c[0];
-        s[0] = prev;
-#pragma unroll 8
-        for (int i = 1; i < m; ++i) {
-            prev = fma(inv_den[i], prev, c[i]);
-            s[i] = prev;
-        }
-        double next = prev;
-#pragma unroll 8
-        for (int i = m - 2; i >= 0; --i) {
-            next = fma(up[i], next, s[i]);
-            s[i] = next;
-        }
-    }
-    __syncthreads();
-    for (int item = threadIdx.x; item < 2 * (n - 1); item += blockDim.x) {
-        const int row = item / (n - 1);
-        const int i = item - row * (n - 1);
-        const double* yy = y + row * n;
-        const double* s = sol + row * n;
-        const double h = x[i + 1] - x[i];
-        const double sl = i == 0 ? 0.0 : s[i - 1];
-        const double sr = i == n - 2 ? 0.0 : s[i];
-        double* c = out + n + (size_t)row * 4 * (n - 1) + 4 * (size_t)i;
-        c[0] = yy[i];
-        c[1] = (yy[i + 1] - yy[i]) / h - h * (2.0 * sl + sr) / 6.0;
-        c[2] = sl / 2.0;
-        c[3] = (sr - sl) / (6.0 * h);
+    double carry = __shfl_up_sync(0xffffffffu, C, 1);
+    if (lane == 0) carry = 0.0;
+    for (int i = begin; i < end; ++i) {
+        const int k = at(i);
+        carry = fma(a[k], carry, c[k]);
+        c[k] = carry;
     }
 }
 
-// Active parents: index > 0 and N <= 0.99999 (bk/evolution.py:501), compacted in
-// index order by a ballot scan, one CTA per set (blockIdx.x).
-__global__ void __launch_bounds__(1024) active_kernel(RowsArg rows, int n, int shard, int shards,
-                                                      int32_t* __restrict__ active, int32_t* __restrict__ count)
+// The active parents of a row (index > 0 and N <= 0.99999, bk/evolution.py:501; index % shards ==
+// shard), compacted in index order by a ballot scan; called by all threads of a CTA.
+__device__ __forceinline__ void compact_active(const double* __restrict__ N, int n, int shard, int shards,
+                                               int32_t* __restrict__ active, int32_t* __restrict__ count)
 {
-    const double* __restrict__ N = rows.at(blockIdx.x);
-    active += (size_t)blockIdx.x * n;
-    count += blockIdx.x;
     __shared__ int warp_counts[32];
     __shared__ int base;
     if (threadIdx.x == 0) base = 0;
@@ -150,6 +80,115 @@ __global__ void __launch_bounds__(1024) active_kernel(RowsArg rows, int n, int s
     if (threadIdx.x == 0) *count = base;
 }
 
+// factor: [2][n] = 1/denominator and upper coefficient of the Thomas sweep for
+// the natural-spline system on the knots log r (it depends on the grid only).
+// With compute_factor set, one warp forms it first (and stores it for later calls).
+// One CTA per set (blockIdx.x): row N.at(set), tables at out + set * spline_doubles(n), its own
+// factorisation copy at factor + set * 2n.  `start` (optional buffers): the active list of
+// the row and the cleared sums of the right-hand side that begins with this refit, which
+// were two more launches and two more memsets on its critical path.
+// What bounds it: the latency of the dependent sweeps (33 us for 400 knots with one thread per
+// row; the scans leave about 8).
+__global__ void __launch_bounds__(256) splines_kernel(const double* __restrict__ r, RowsArg rows,
+                                                      int n, int force_positive, double* __restrict__ factor,
+                                                      int compute_factor, double* __restrict__ out, RhsStart start)
+{
+    const double* __restrict__ N = rows.at(blockIdx.x);
+    factor += (size_t)blockIdx.x * 2 * n;
+    out += (size_t)blockIdx.x * spline_doubles(n);
+    extern __shared__ double smem[];
+    double* x = smem;             // [n]
+    double* y = x + n;            // [2][n]
+    double* sol = y + 2 * n;      // [2][n]
+    double* low = sol + 2 * n;    // [n]
+    double* up = low + n;         // [n]
+    const int m = n - 2;
+    for (int i = threadIdx.x; i < n; i += blockDim.x) {
+        x[i] = log(r[i]);
+        out[i] = x[i];
+        const double v = N[i];
+        // log N row: N > 1 -> 1; force_positive: N < 0 -> 0
+        double vn = v > 1.0 ? 1.0 : v;
+        if (force_positive && vn < 0.0) vn = 0.0;
+        y[i] = vn > 0.0 ? log(vn) : kMinLog;
+        // log S row: S = 1 - N; S < 0 -> 0; force_positive: S > 1 -> 1
+        double ns = v;
+        if (force_positive && ns < 0.0) ns = 0.0;
+        y[n + i] = ns < 1.0 ? log1p(-ns) : kMinLog;
+        if (start.k1) start.k1[(size_t)blockIdx.x * n + i] = 0.0;
+    }
+    if (start.k2kf)
+        for (int i = threadIdx.x; i < 3 * n; i += blockDim.x) start.k2kf[(size_t)blockIdx.x * 3 * n + i] = 0.0;
+    __syncthreads();
+    if (compute_factor && threadIdx.x < 32 && m >= 1) {
+        // denominators of the forward sweep (interpolation.py:124-149): lane l its own stretch,
+        // entered kFactorWarmup elements earlier from the undivided denominator.  The recurrence
+        // forgets its start (a factor of 0.07 a step on the uniform grid, under 0.45 on any), so
+        // the stretch is the serial sweep's to the last digits.
+        constexpr int kFactorWarmup = 48;
+        const int per = (m + 31) / 32;
+        const int begin = min((int)threadIdx.x * per, m), end = min(begin + per, m);
+        int i = max(0, begin - kFactorWarmup);
+        double inv = 1.0 / (2.0 * ((x[i + 1] - x[i]) + (x[i + 2] - x[i + 1])));
+        if (i == begin && begin < end) factor[i] = inv;
+        for (++i; i < end; ++i) {
+            const double h = x[i + 1] - x[i];
+            const double upper_prev = h * inv;
+            if (i > begin || begin == 0) factor[n + i - 1] = upper_prev;
+            inv = 1.0 / (2.0 * (h + (x[i + 2] - x[i + 1])) - h * upper_prev);
+            if (i >= begin) factor[i] = inv;
+        }
+        if (begin < end && end < m) factor[n + end - 1] = (x[end + 1] - x[end]) * inv;
+    }
+    __syncthreads();
+    // The forward sweep s_i = (b_i - h_i s_{i-1}) / d_i as s_i = c_i + a_i s_{i-1} with
+    // c_i = b_i / d_i and a_i = -h_i / d_i; the back substitution likewise with the negated
+    // upper diagonal.
+    for (int item = threadIdx.x; item < 2 * m; item += blockDim.x) {
+        const int row = item / m, i = item - row * m;
+        const double* yy = y + row * n;
+        sol[row * n + i] =
+            6.0 * ((yy[i + 2] - yy[i + 1]) / (x[i + 2] - x[i + 1]) - (yy[i + 1] - yy[i]) / (x[i + 1] - x[i])) * factor[i];
+        if (row == 0) {
+            low[i] = i > 0 ? -(x[i + 1] - x[i]) * factor[i] : 0.0;
+            up[i] = i < m - 1 ? -factor[n + i] : 0.0;
+        }
+    }
+    __syncthreads();
+    // warp 0 solves row 0, warp 1 row 1
+    if (threadIdx.x < 64 && m >= 1) {
+        double* s = sol + (threadIdx.x >> 5) * n;
+        warp_affine_scan<false>(low, s, m);
+        __syncwarp();
+        warp_affine_scan<true>(up, s, m);
+    }
+    __syncthreads();
+    for (int item = threadIdx.x; item < 2 * (n - 1); item += blockDim.x) {
+        const int row = item / (n - 1);
+        const int i = item - row * (n - 1);
+        const double* yy = y + row * n;
+        const double* s = sol + row * n;
+        const double h = x[i + 1] - x[i];
+        const double sl = i == 0 ? 0.0 : s[i - 1];
+        const double sr = i == n - 2 ? 0.0 : s[i];
+        double* c = out + n + (size_t)row * 4 * (n - 1) + 4 * (size_t)i;
+        c[0] = yy[i];
+        c[1] = (yy[i + 1] - yy[i]) / h - h * (2.0 * sl + sr) / 6.0;
+        c[2] = sl / 2.0;
+        c[3] = (sr - sl) / (6.0 * h);
+    }
+    if (start.active)
+        compact_active(N, n, start.shard, start.shards, start.active + (size_t)blockIdx.x * n,
+                       start.count + blockIdx.x);
+}
+
+// The active list alone, one CTA per set (blockIdx.x).
+__global__ void __launch_bounds__(1024) active_kernel(RowsArg rows, int n, int shard, int shards,
+                                                      int32_t* __restrict__ active, int32_t* __restrict__ count)
+{
+    compact_active(rows.at(blockIdx.x), n, shard, shards, active + (size_t)blockIdx.x * n, count + blockIdx.x);
+}
+
 template <typename T>
 __global__ void sobol_draw_kernel(SobolDirsArg dirs, uint64_t offset, uint64_t n, T* __restrict__ out)
 {
@@ -164,14 +203,14 @@ __global__ void sobol_draw_kernel(SobolDirsArg dirs, uint64_t offset, uint64_t n
 }
 
 cudaError_t launch_splines(const double* r, const RowsArg& N, int n, int sets, int force_positive, double* factor,
-                           int compute_factor, double* out, cudaStream_t stream)
+                           int compute_factor, double* out, cudaStream_t stream, const RhsStart& start)
 {
-    const size_t smem = sizeof(double) * 9 * (size_t)n;
+    const size_t smem = sizeof(double) * 7 * (size_t)n;
     if (smem > 48 * 1024) {
         cudaError_t e = raise_dynamic_smem((const void*)splines_kernel, smem);
         if (e != cudaSuccess) return e;
     }
-    splines_kernel<<<sets, 256, smem, stream>>>(r, N, n, force_positive, factor, compute_factor, out);
+    splines_kernel<<<sets, 256, smem, stream>>>(r, N, n, force_positive, factor, compute_factor, out, start);
     return cudaGetLastError();
 }
 
