@@ -12,6 +12,7 @@ import ctypes
 import threading
 from pathlib import Path
 
+import numpy as np
 import torch
 
 from nlo_bk_optimized_b200 import build as _build
@@ -347,14 +348,12 @@ def sobol_dirs(dims: int, seed: int) -> SobolDirs:
     """Direction numbers of SobolEngine(dims, scramble=True, seed)."""
 
     engine = torch.quasirandom.SobolEngine(dims, scramble=True, seed=seed)
-    state = engine.sobolstate.tolist()
-    shift = engine.shift.tolist()
     dirs = SobolDirs()
     dirs.dims = dims
-    for d in range(dims):
-        for j in range(30):
-            dirs.state[d][j] = int(state[d][j])
-        dirs.shift[d] = int(shift[d])
+    state = engine.sobolstate.numpy().astype(np.uint32)
+    shift = engine.shift.numpy().astype(np.uint32)
+    ctypes.memmove(ctypes.byref(dirs, SobolDirs.state.offset), state.ctypes.data, state.nbytes)
+    ctypes.memmove(ctypes.byref(dirs, SobolDirs.shift.offset), shift.ctypes.data, shift.nbytes)
     return dirs
 
 

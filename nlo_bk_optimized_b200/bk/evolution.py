@@ -215,7 +215,7 @@ def rhs(
     points = r64.numel()
     prec = precision if precision is not None else precision_of(config, r.dtype)
     params = params_of(config, prec)
-    lower, width = nlo_box(float(r64[0]), float(r64[-1]))
+    lower, width = nlo_box(*r64[:: points - 1].tolist())
     dirs = _native.sobol_dirs(4, 0 if seed is None else seed)
     box = _native.box(lower, width)
     dndy = torch.empty_like(N64)
@@ -365,7 +365,7 @@ def _evolve_rows(
     points = r64.numel()
     status = torch.zeros(1, dtype=torch.int32, device=device)
     params = params_of(config, precision)
-    lower, width = nlo_box(float(r64[0]), float(r64[-1]))
+    lower, width = nlo_box(*r64[:: points - 1].tolist())
     box = _native.box(lower, width)
     opts, dirs_all = vegas_evolution_setup(config, seed)
     dirs = dirs_all[0]
@@ -535,9 +535,10 @@ def compute_dndy(
     # the history of the initial rapidity alone (bk/evolution.py:76-79)
     history = (torch.zeros(1, dtype=torch.float64, device=device), N.unsqueeze(0))
     _, K1, K2_Kf = rhs(N, r64, config, seed=seed, precision=precision_of(config, dtype), history=history)
-    keep = (torch.arange(r64.numel(), device=device) > 0) & (N <= 0.99999)
-    return DNDYResult(r=r64[keep].to(dtype), K1=K1[keep].to(dtype), K2_Kf=K2_Kf[keep].to(dtype),
-                      N=N[keep].to(dtype))
+    keep = N <= 0.99999
+    keep[0] = False
+    kept = torch.stack((r64, K1, K2_Kf, N))[:, keep].to(dtype)
+    return DNDYResult(*(row.contiguous() for row in kept))
 
 
 __all__ = ["AdaptiveRK2", "DNDYResult", "bk_steps", "compute_dndy", "evolve_table", "nlo_box", "rhs", "solve_bk",

@@ -42,7 +42,6 @@ from nlo_bk_optimized_b200.numerics.integration import (
     VegasOptions,
     budget_options,
     gauss_legendre_terms,
-    state_results,
     vegas_terms,
 )
 
@@ -107,17 +106,29 @@ def _validate_kinematics(Q2: torch.Tensor, xbj: torch.Tensor) -> None:
         raise ValueError("Q2 must be positive and xbj must lie in (0, 1]")
 
 
-def _scale_result(result: IntegralResult, factor: float) -> IntegralResult:
-    return IntegralResult(result.value * factor, result.error * abs(factor), result.n_eval, result.converged,
-                          result.seed)
+@dataclass(frozen=True, slots=True)
+class _Sum:
+    """An IntegralResult in plain numbers: what the results of many jobs are combined in."""
+
+    value: float
+    error: float
+    n_eval: int
+    converged: bool
+    seed: int | None = None
+
+    def scaled(self, factor: float) -> "_Sum":
+        return _Sum(self.value * factor, self.error * abs(factor), self.n_eval, self.converged, self.seed)
+
+    def result(self, device: torch.device) -> IntegralResult:
+        value, error = torch.tensor((self.value, self.error), dtype=torch.float64, device=device).unbind()
+        return IntegralResult(value, error, self.n_eval, self.converged, self.seed)
 
 
-def _sum_results(results, seed: int | None) -> IntegralResult:
+def _sum_results(results, seed: int | None) -> _Sum:
     if not results:
         raise ValueError("at least one integration result is required")
-    value = torch.stack([r.value for r in results]).sum()
-    error = torch.sqrt(torch.stack([r.error.square() for r in results]).sum())
-    return IntegralResult(value, error, sum(r.n_eval for r in results), all(r.converged for r in results), seed)
+    return _Sum(sum(r.value for r in results), math.sqrt(sum(r.error * r.error for r in results)),
+                sum(r.n_eval for r in results), all(r.converged for r in results), seed)
 
 
 def dipole_rapidity(Q2: float, xbj: float, mf: float, scheme: HeavyQuarkX) -> float:
@@ -168,13 +179,13 @@ class _Engine:
         return None, [j.dipole.native() for j in group]
 
     def run(self) -> None:
+        from nlo_bk_optimized_b200.dis.fixed_sobol import FIXED_SOBOL_EVALUATIONS, fixed_sobol_device
+
         precision = _precision(self.config)
         pending = []
         todo = [j for j in self.jobs if not j.done]
         for job in todo:
             if job.fixed is not None:
-                from nlo_bk_optimized_b200.dis.fixed_sobol import FIXED_SOBOL_EVALUATIONS, fixed_sobol_device
-
                 pol, quark = job.fixed
                 _, est = fixed_sobol_device(job.kin.Q2, job.kin.xbj, pol, quark, job.dipole, self.config,
                                             seed=job.seed, device=self.device, precision=precision)
@@ -210,12 +221,15 @@ class _Engine:
             native, natives = self._natives(group)
             state = vegas_terms(term, [j.kin for j in group], native, options, [j.seed for j in group],
                                 precision=precision, device=self.device, dipoles=natives)
-            pending.append(("vegas", group, state_results(state, term, options.bins)))
-        for kind, group, out in pending:
+            pending.append(("vegas", group, state[:, _native.DIS_DIMS[term] * (options.bins + 1) :]))
+        # one read-back for every group's results
+        flat = [out.reshape(-1) for _, _, out in pending]
+        host = torch.cat(flat).tolist() if flat else []
+        for (kind, group, out), values in zip(pending, _split(host, flat)):
             for job in group:
                 job.done = True
             if kind == "fixed":
-                est = out.cpu()
+                est = torch.tensor(values, dtype=torch.float64).reshape(out.shape)
                 job = group[0]
                 totals = est.sum(dim=1)
                 job.value = float(totals.mean())
@@ -223,27 +237,29 @@ class _Engine:
                 job.n_eval = FIXED_SOBOL_EVALUATIONS
                 job.converged = job.error <= self.config.epsrel * abs(job.value)
             elif kind == "gl":
-                host = out.cpu()
                 for j, job in enumerate(group):
-                    job.value = float(host[j, 0])
-                    job.error = float(host[j, 1])
+                    job.value, job.error = values[2 * j : 2 * j + 2]
                     n = job.points
                     job.n_eval = n * n + max(2, n // 2) ** 2
                     job.converged = job.error <= self.config.epsrel * abs(job.value)
             else:
-                value, error = out["value"].cpu(), out["error"].cpu()
-                evals, conv = out["n_eval"].cpu(), out["converged"].cpu()
+                slots = out.shape[1]
                 for j, job in enumerate(group):
-                    job.value = float(value[j])
-                    job.error = float(error[j])
-                    job.n_eval = int(evals[j])
-                    job.converged = bool(conv[j] != 0)
+                    row = values[slots * j : slots * (j + 1)]
+                    job.value, job.error = row[_native.VEGAS_VALUE], row[_native.VEGAS_ERROR]
+                    job.n_eval = int(row[_native.VEGAS_EVALS])
+                    job.converged = row[_native.VEGAS_CONVERGED] != 0
 
 
-def _result(job: _Job, scale: float, device: torch.device, seed) -> IntegralResult:
-    return IntegralResult(torch.tensor(job.value * scale, dtype=torch.float64, device=device),
-                          torch.tensor(job.error * abs(scale), dtype=torch.float64, device=device),
-                          job.n_eval, job.converged, seed)
+def _split(values: list[float], tensors: list[torch.Tensor]):
+    start = 0
+    for t in tensors:
+        yield values[start : start + t.numel()]
+        start += t.numel()
+
+
+def _result(job: _Job, scale: float) -> _Sum:
+    return _Sum(job.value, job.error, job.n_eval, job.converged).scaled(scale)
 
 
 def _lo_Y(dipole: Dipole, xbj: float) -> float:
@@ -315,7 +331,9 @@ def _plan_lo(engine: _Engine, Q2: float, xbj: float, pol: Polarization, points: 
              dipole: Dipole | None = None) -> _Job:
     dipole = dipole if dipole is not None else engine.dipole
     kin = kinematics(Q2, xbj, pol, engine.config)
-    return engine.add(_Job(TERMS["LO"], kin, points=points, lo_Y=_lo_Y(dipole, xbj), dipole=dipole))
+    # only a table is initialised at its rapidity; the LO jobs of a GBW dipole are one group
+    lo_Y = _lo_Y(dipole, xbj) if isinstance(dipole, BKDipole) else None
+    return engine.add(_Job(TERMS["LO"], kin, points=points, lo_Y=lo_Y, dipole=dipole))
 
 
 def _plan_sigma(engine: _Engine, Q2: float, xbj: float, pol: Polarization, *, seed: int, points: int,
@@ -360,21 +378,28 @@ def _run_with_fallback(engine: _Engine, plans: list[_SigmaPlan]) -> None:
         engine.run()
 
 
-def _sigma_result(plan: _SigmaPlan, config: DISConfig, device: torch.device) -> IntegralResult:
-    lo = _result(plan.lo, LO_FACTOR, device, None)
+def _sigma_result(plan: _SigmaPlan, config: DISConfig) -> _Sum:
+    lo = _result(plan.lo, LO_FACTOR)
     if config.order is DISOrder.LO:
         return lo
     seed = plan.seed
-    per_quark = [_sum_results([_result(j, q.charge**2, device, None) for j in jobs], seed)
-                 for q, jobs in zip(config.quarks, plan.dip)]
-    dip = _scale_result(_sum_results(per_quark, seed), DIP_FACTOR)
-    if plan.qg_fixed:
-        per_quark = [_result(j, q.charge**2, device, None) for q, j in zip(config.quarks, plan.qg_fixed)]
-    else:
-        per_quark = [_sum_results([_result(j, q.charge**2, device, None) for j in jobs], seed + 100)
-                     for q, jobs in zip(config.quarks, plan.qg)]
-    qg = _scale_result(_sum_results(per_quark, seed + 100), QG_FACTOR)
+    dip = _dip_result(plan, config, seed).scaled(DIP_FACTOR)
+    qg = _qg_result(plan, config, seed + 100).scaled(QG_FACTOR)
     return _sum_results((lo, dip, qg), seed)
+
+
+def _dip_result(plan: _SigmaPlan, config: DISConfig, seed: int) -> _Sum:
+    return _sum_results([_sum_results([_result(j, q.charge**2) for j in jobs], seed)
+                         for q, jobs in zip(config.quarks, plan.dip)], seed)
+
+
+def _qg_result(plan: _SigmaPlan, config: DISConfig, seed: int) -> _Sum:
+    if plan.qg_fixed:
+        per_quark = [_result(j, q.charge**2) for q, j in zip(config.quarks, plan.qg_fixed)]
+    else:
+        per_quark = [_sum_results([_result(j, q.charge**2) for j in jobs], seed)
+                     for q, jobs in zip(config.quarks, plan.qg)]
+    return _sum_results(per_quark, seed)
 
 
 def _sf_factor(Q2: float, config: DISConfig) -> float:
@@ -391,7 +416,7 @@ def photon_proton_cross_section_LO_d2b(Q2: torch.Tensor, xbj: torch.Tensor, pola
     engine = _Engine(dipole, config, _device(Q2))
     job = _plan_lo(engine, float(Q2), float(xbj), polarization, quadrature_points)
     engine.run()
-    return _result(job, LO_FACTOR, engine.device, None)
+    return _result(job, LO_FACTOR).result(engine.device)
 
 
 def sigma_dip_d2b(Q2: torch.Tensor, xbj: torch.Tensor, polarization: Polarization, dipole: Dipole,
@@ -404,9 +429,7 @@ def sigma_dip_d2b(Q2: torch.Tensor, xbj: torch.Tensor, polarization: Polarizatio
                        overrides=_integration_overrides(options))
     engine.jobs = [j for jobs in plan.dip for j in jobs]
     engine.run()
-    per_quark = [_sum_results([_result(j, q.charge**2, engine.device, None) for j in jobs], seed)
-                 for q, jobs in zip(config.quarks, plan.dip)]
-    return _scale_result(_sum_results(per_quark, seed), DIP_FACTOR)
+    return _dip_result(plan, config, seed).scaled(DIP_FACTOR).result(engine.device)
 
 
 def sigma_qg_d2b(Q2: torch.Tensor, xbj: torch.Tensor, polarization: Polarization, dipole: Dipole,
@@ -418,12 +441,7 @@ def sigma_qg_d2b(Q2: torch.Tensor, xbj: torch.Tensor, polarization: Polarization
                        overrides=_integration_overrides(options), fixed=Q2.dtype == torch.float32)
     engine.jobs = list(plan.qg_fixed) + [j for jobs in plan.qg for j in jobs]
     _run_with_fallback(engine, [plan])
-    if plan.qg_fixed:
-        per_quark = [_result(j, q.charge**2, engine.device, None) for q, j in zip(config.quarks, plan.qg_fixed)]
-    else:
-        per_quark = [_sum_results([_result(j, q.charge**2, engine.device, None) for j in jobs], seed)
-                     for q, jobs in zip(config.quarks, plan.qg)]
-    return _scale_result(_sum_results(per_quark, seed), QG_FACTOR)
+    return _qg_result(plan, config, seed).scaled(QG_FACTOR).result(engine.device)
 
 
 def photon_proton_cross_section_d2b(Q2: torch.Tensor, xbj: torch.Tensor, polarization: Polarization,
@@ -434,22 +452,24 @@ def photon_proton_cross_section_d2b(Q2: torch.Tensor, xbj: torch.Tensor, polariz
     plan = _plan_sigma(engine, float(Q2), float(xbj), polarization, seed=seed, points=quadrature_points,
                        overrides=_integration_overrides(options), fixed=Q2.dtype == torch.float32)
     _run_with_fallback(engine, [plan])
-    return _sigma_result(plan, config, engine.device)
+    return _sigma_result(plan, config).result(engine.device)
 
 
 def FL(Q2: torch.Tensor, xbj: torch.Tensor, dipole: Dipole, config: DISConfig, **integration_options) -> IntegralResult:
     sigma = photon_proton_cross_section_d2b(Q2, xbj, Polarization.L, dipole, config, **integration_options)
-    return _scale_result(sigma, _sf_factor(float(Q2), config))
+    factor = _sf_factor(float(Q2), config)
+    return IntegralResult(sigma.value * factor, sigma.error * abs(factor), sigma.n_eval, sigma.converged, sigma.seed)
 
 
 def FT(Q2: torch.Tensor, xbj: torch.Tensor, dipole: Dipole, config: DISConfig, **integration_options) -> IntegralResult:
     sigma = photon_proton_cross_section_d2b(Q2, xbj, Polarization.T, dipole, config, **integration_options)
-    return _scale_result(sigma, _sf_factor(float(Q2), config))
+    factor = _sf_factor(float(Q2), config)
+    return IntegralResult(sigma.value * factor, sigma.error * abs(factor), sigma.n_eval, sigma.converged, sigma.seed)
 
 
 def _two_polarisations(Q2: torch.Tensor, xbj: torch.Tensor, dipole: Dipole, config: DISConfig,
-                       options: dict) -> tuple[IntegralResult, IntegralResult]:
-    """F_T and F_L of one point in one engine run, with F2's seed rule (F_L gets seed + 1000
+                       options: dict) -> tuple[_Sum, _Sum, torch.device]:
+    """F_T and F_L of one point (and their device) in one engine run, with F2's seed rule (F_L gets seed + 1000
     when a seed is given, dis/observables.py:581-599)."""
     _validate_kinematics(Q2, xbj)
     options_T = dict(options)
@@ -464,12 +484,13 @@ def _two_polarisations(Q2: torch.Tensor, xbj: torch.Tensor, dipole: Dipole, conf
                                  fixed=Q2.dtype == torch.float32))
     _run_with_fallback(engine, plans)
     factor = _sf_factor(float(Q2), config)
-    return tuple(_scale_result(_sigma_result(p, config, engine.device), factor) for p in plans)
+    sum_T, sum_L = (_sigma_result(p, config).scaled(factor) for p in plans)
+    return sum_T, sum_L, engine.device
 
 
 def F2(Q2: torch.Tensor, xbj: torch.Tensor, dipole: Dipole, config: DISConfig, **integration_options) -> IntegralResult:
-    result_T, result_L = _two_polarisations(Q2, xbj, dipole, config, integration_options)
-    return _sum_results((result_T, result_L), integration_options.get("seed"))
+    result_T, result_L, device = _two_polarisations(Q2, xbj, dipole, config, integration_options)
+    return _sum_results((result_T, result_L), integration_options.get("seed")).result(device)
 
 
 def reduced_cross_section_y(Q2: float, xbj: float, sqrt_s: float) -> float:
@@ -480,13 +501,26 @@ def sigma_r(Q2: torch.Tensor, xbj: torch.Tensor, dipole: Dipole, config: DISConf
             **integration_options) -> IntegralResult:
     """Reduced cross section sigma_r = F2 - y^2/(1 + (1-y)^2) F_L with y = Q^2/(s x_Bj)
     (no counterpart in the reference package, which stops at F2 and F_L)."""
-    result_T, result_L = _two_polarisations(Q2, xbj, dipole, config, integration_options)
+    result_T, result_L, device = _two_polarisations(Q2, xbj, dipole, config, integration_options)
     y = reduced_cross_section_y(float(Q2), float(xbj), sqrt_s)
     f = y * y / (1 + (1 - y) ** 2)
-    value = result_T.value + (1 - f) * result_L.value
-    error = torch.sqrt(result_T.error.square() + ((1 - f) * result_L.error).square())
-    return IntegralResult(value, error, result_T.n_eval + result_L.n_eval,
-                          result_T.converged and result_L.converged, integration_options.get("seed"))
+    return _sum_results((result_T, result_L.scaled(1 - f)), integration_options.get("seed")).result(device)
+
+
+def _structure_columns(plans, Q2: list[float], config: DISConfig) -> dict[str, torch.Tensor]:
+    """F_T, F_L, F_2 and their errors of the points' (T, L) plans, on the host."""
+    rows = []
+    for (pt, pl), q2 in zip(plans, Q2):
+        factor = _sf_factor(q2, config)
+        rt, rl = _sigma_result(pt, config).scaled(factor), _sigma_result(pl, config).scaled(factor)
+        rows.append((rt.value, rl.value, rt.value + rl.value, rt.error, rl.error, math.hypot(rt.error, rl.error)))
+    columns = torch.tensor(rows, dtype=torch.float64).reshape(len(rows), 6).T
+    return dict(zip(("FT", "FL", "F2", "FT_error", "FL_error", "F2_error"), columns))
+
+
+def _to_device(columns: dict[str, torch.Tensor], device: torch.device) -> dict[str, torch.Tensor]:
+    rows = torch.stack(tuple(columns.values())).to(device)
+    return {k: row.clone() for k, row in zip(columns, rows)}
 
 
 def structure_functions(Q2: torch.Tensor, xbj: torch.Tensor, dipole: Dipole, config: DISConfig, *,
@@ -514,22 +548,13 @@ def structure_functions(Q2: torch.Tensor, xbj: torch.Tensor, dipole: Dipole, con
                       _plan_sigma(engine, q2, x, Polarization.L, seed=seed + 1000, points=quadrature_points,
                                   overrides=overrides, fixed=fixed)))
     _run_with_fallback(engine, [p for pair in plans for p in pair])
-    out = {k: torch.empty(Q2h.numel(), dtype=torch.float64) for k in ("FT", "FL", "F2", "FT_error", "FL_error",
-                                                                      "F2_error")}
-    for i, (pt, pl) in enumerate(plans):
-        factor = _sf_factor(float(Q2h[i]), config)
-        rt = _scale_result(_sigma_result(pt, config, torch.device("cpu")), factor)
-        rl = _scale_result(_sigma_result(pl, config, torch.device("cpu")), factor)
-        out["FT"][i], out["FL"][i] = rt.value, rl.value
-        out["FT_error"][i], out["FL_error"][i] = rt.error, rl.error
-        out["F2"][i] = rt.value + rl.value
-        out["F2_error"][i] = math.hypot(float(rt.error), float(rl.error))
+    out = _structure_columns(plans, Q2h.tolist(), config)
     if sqrt_s is not None:
         y = Q2h / (sqrt_s**2 * xh)
         f = y * y / (1 + (1 - y) ** 2)
         out["sigma_r"] = out["FT"] + (1 - f) * out["FL"]
         out["sigma_r_error"] = torch.sqrt(out["FT_error"] ** 2 + ((1 - f) * out["FL_error"]) ** 2)
-    return {k: v.to(device) for k, v in out.items()}
+    return _to_device(out, device)
 
 
 def structure_functions_many(Q2, xbj, dipoles, config: DISConfig, *, sqrt_s: float | None = None, seed: int = 0,
@@ -567,22 +592,14 @@ def structure_functions_many(Q2, xbj, dipoles, config: DISConfig, *, sqrt_s: flo
                       _plan_sigma(engine, q2, x, Polarization.L, seed=sd + 1000, points=quadrature_points,
                                   overrides=overrides, fixed=fixed, dipole=d)))
     _run_with_fallback(engine, [p for pair in plans for p in pair])
-    out = {k: torch.empty(n, dtype=torch.float64) for k in ("FT", "FL", "F2", "FT_error", "FL_error", "F2_error")}
-    for i, (pt, pl) in enumerate(plans):
-        factor = _sf_factor(Q2h[i], config)
-        rt = _scale_result(_sigma_result(pt, config, torch.device("cpu")), factor)
-        rl = _scale_result(_sigma_result(pl, config, torch.device("cpu")), factor)
-        out["FT"][i], out["FL"][i] = rt.value, rl.value
-        out["FT_error"][i], out["FL_error"][i] = rt.error, rl.error
-        out["F2"][i] = rt.value + rl.value
-        out["F2_error"][i] = math.hypot(float(rt.error), float(rl.error))
+    out = _structure_columns(plans, Q2h, config)
     if sqrt_s is not None:
         q2t, xt = torch.tensor(Q2h, dtype=torch.float64), torch.tensor(xh, dtype=torch.float64)
         y = q2t / (sqrt_s**2 * xt)
         f = y * y / (1 + (1 - y) ** 2)
         out["sigma_r"] = out["FT"] + (1 - f) * out["FL"]
         out["sigma_r_error"] = torch.sqrt(out["FT_error"] ** 2 + ((1 - f) * out["FL_error"]) ** 2)
-    return {k: v.to(device) for k, v in out.items()}
+    return _to_device(out, device)
 
 
 def structure_function_batch(points, dipole: Dipole, config: DISConfig, *, quadrature_points: int = 24,
@@ -604,7 +621,7 @@ def structure_function_batch(points, dipole: Dipole, config: DISConfig, *, quadr
     plans = [_plan_sigma(engine, q2, x, pol, seed=seed, points=quadrature_points, overrides=overrides,
                          fixed=single_precision) for q2, x, pol, seed in points]
     _run_with_fallback(engine, plans)
-    return [_scale_result(_sigma_result(plan, config, device), _sf_factor(q2, config))
+    return [_sigma_result(plan, config).scaled(_sf_factor(q2, config)).result(device)
             for plan, (q2, _, _, _) in zip(plans, points)]
 
 
