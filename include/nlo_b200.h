@@ -255,7 +255,7 @@ int nlo_bk_evolve_history(const nlo_bk_params* params, const double* r, int32_t 
  * tables: host array of `sets` device pointers, each a double[(steps+1)*points] table whose
  * row 0 holds the set's initial row.  dirs: host array of `sets` Sobol direction sets (at
  * least 4 dimensions each).  samples: host int64[sets], each 0..2^30.  waves (1..64): K2+Kf
- * CTAs per launch ~ waves x 2 x SM count, spread over the sets' groups.  status: device
+ * CTAs per launch ~ waves x 3 x SM count, each set's share by its budget.  status: device
  * uint32[sets], reset and then flagged per set as in nlo_bk_evolve.  The kinematical
  * constraint is not accepted. */
 size_t nlo_bk_sets_workspace_bytes(int32_t points, int32_t sets, int32_t waves);

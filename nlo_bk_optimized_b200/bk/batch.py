@@ -2,14 +2,12 @@
 
 All sets of a call advance together through one ``nlo_bk_evolve_sets`` call (the whole
 rapidity loop in C, no host synchronisation): every stage is one launch per kernel for all
-sets, and the K2+Kf launch gives its lanes (set, parent) pairs -- a CTA stages one tile of
-sample records per set it holds, and sets of equal budget share CTAs, so small budgets no
-longer pay a whole under-filled launch each.  Each set has its own Sobol seed (a set of budget
-S uses the first S points of its sequence).  The K2+Kf launch takes about ``waves`` x 2 CTAs
-per SM, spread over the sets' groups -- which fixes the sample chunk each CTA sweeps -- and
-``tune_waves`` picks ``waves`` by timing one rapidity step of a sample of the sets at each
-candidate.  A set's rows equal ``solve_bk``'s for the same initial row, budget and seed up to
-the order in which the FP64 partial sums of the CTAs are added.
+sets, and the K2+Kf launch gives every set CTAs in proportion to its budget, so small budgets
+do not pay a whole under-filled launch each.  Each set has its own Sobol seed (a set of budget
+S uses the first S points of its sequence).  The K2+Kf launch takes about ``waves`` x 3 CTAs
+per SM, and ``tune_waves`` picks ``waves`` by timing one rapidity step of a sample of the sets
+at each candidate.  A set's rows equal ``solve_bk``'s for the same initial row, budget and seed
+up to the order in which the FP64 partial sums of the CTAs are added.
 """
 
 from __future__ import annotations

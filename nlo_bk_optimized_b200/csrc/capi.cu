@@ -6,7 +6,6 @@
 
 #include <cmath>
 #include <cstdio>
-#include <algorithm>
 #include <cstddef>
 #include <cstring>
 #include <map>
@@ -864,14 +863,8 @@ int nlo_bk_evolve_sets(const nlo_bk_params* params, const double* r, int32_t poi
     double* tmp = stage + 4 * S * n;
     double* cur = stage + 5 * S * n;
 
-    // slots in order of decreasing budget (ties by set index), so that slot 0 of every group
-    // holds the group's largest budget and sets of one budget share CTAs
-    int32_t order[kMaxSets];
-    for (int i = 0; i < sets; ++i) order[i] = i;
-    std::stable_sort(order, order + sets, [&](int32_t a, int32_t b) { return samples[a] > samples[b]; });
-    const int slots = L.groups * L.per_cta;
-    int32_t slot_set[kMaxSlots];
-    for (int q = 0; q < slots; ++q) slot_set[q] = q < sets ? order[q] : -1;
+    uint16_t cta_first[kMaxSets + 1];
+    sets_ctas(L, params->precision == NLO_PRECISION_FP64, points, samples, sets, cta_first);
     const bool nlo = order_has_nlo(params->order);
     std::vector<SobolDirsArg> set_dirs(sets);
     const SobolDirsArg* dir_ptrs[kMaxSets];
@@ -879,7 +872,7 @@ int nlo_bk_evolve_sets(const nlo_bk_params* params, const double* r, int32_t poi
         set_dirs[i] = to_arg(dirs + i);
         dir_ptrs[i] = &set_dirs[i];
     }
-    cudaError_t e = launch_sets_setup(tables, samples, slot_set, dir_ptrs, sets, slots, nlo, table, s);
+    cudaError_t e = launch_sets_setup(tables, samples, cta_first, dir_ptrs, sets, nlo, table, s);
     if (e != cudaSuccess) return cuda_fail(e, "sets setup");
     if ((e = cudaMemsetAsync(status, 0, sizeof(uint32_t) * S, s)) != cudaSuccess) return cuda_fail(e, "status reset");
     double* const* rows = reinterpret_cast<double* const*>(base + off[8] + offsetof(SetTable, rows));
@@ -920,8 +913,8 @@ int nlo_bk_evolve_sets(const nlo_bk_params* params, const double* r, int32_t poi
                 cudaSuccess)
                 return cuda_fail(e, "k1");
             if (beside && (e = cudaEventRecord(side.join, side.aux)) != cudaSuccess) return cuda_fail(e, "join");
-            if (nlo && (e = launch_k2kf_sets(*params, r, points, sets, spline, spline_doubles(points), active, counts,
-                                             *box, L, table, k2kf, partial, s, true)) != cudaSuccess)
+            if (nlo && (e = launch_k2kf_sets(*params, r, points, sets, spline, active, counts, *box,
+                                             cta_first[sets], table, k2kf, partial, s, true)) != cudaSuccess)
                 return cuda_fail(e, "k2kf sets");
             if (beside && (e = cudaStreamWaitEvent(s, side.join, 0)) != cudaSuccess) return cuda_fail(e, "join");
             return (int)NLO_OK;

@@ -93,8 +93,8 @@ __global__ void axpy_sets_kernel(RowsArg N, StageArgs a, int n, RowsArg out, int
 struct SetupArg {
     double* rows[kMaxSets];
     uint32_t samples[kMaxSets];
-    int16_t slot_set[kMaxSlots];
-    int sets, slots, nlo;
+    uint16_t cta_first[kMaxSets + 1];
+    int sets, nlo;
 };
 static_assert(sizeof(SetupArg) <= 4096, "the set table travels as a kernel parameter");
 
@@ -120,28 +120,25 @@ __global__ void sets_setup_kernel(SetupArg a, SetTable* __restrict__ t)
         t->samples[i] = i < a.sets ? a.samples[i] : 0u;
         t->inv[i] = i < a.sets && a.nlo && a.samples[i] > 0 ? 1.0 / (double)a.samples[i] : 0.0;
     }
-    if (i < kMaxSlots) t->slot_set[i] = i < a.slots ? (int32_t)a.slot_set[i] : -1;
-    __syncthreads();
-    if (i < a.slots && t->slot_set[i] >= 0) t->set_slot[t->slot_set[i]] = i;
+    if (i <= a.sets) t->cta_first[i] = a.cta_first[i];
 }
 
 }  // namespace
 
-cudaError_t launch_sets_setup(double* const* rows, const int64_t* samples, const int32_t* slot_set,
-                              const SobolDirsArg* const* dirs, int sets, int slots, bool nlo, SetTable* table,
+cudaError_t launch_sets_setup(double* const* rows, const int64_t* samples, const uint16_t* cta_first,
+                              const SobolDirsArg* const* dirs, int sets, bool nlo, SetTable* table,
                               cudaStream_t stream)
 {
-    if (sets < 1 || sets > kMaxSets || slots < sets || slots > kMaxSlots) return cudaErrorInvalidValue;
+    if (sets < 1 || sets > kMaxSets) return cudaErrorInvalidValue;
     SetupArg a;
     for (int i = 0; i < kMaxSets; ++i) {
         a.rows[i] = i < sets ? rows[i] : nullptr;
         a.samples[i] = i < sets ? (uint32_t)samples[i] : 0u;
     }
-    for (int i = 0; i < kMaxSlots; ++i) a.slot_set[i] = (int16_t)(i < slots ? slot_set[i] : -1);
+    for (int i = 0; i <= kMaxSets; ++i) a.cta_first[i] = i <= sets ? cta_first[i] : (uint16_t)0;
     a.sets = sets;
-    a.slots = slots;
     a.nlo = nlo ? 1 : 0;
-    sets_setup_kernel<<<1, (kMaxSlots + 31) / 32 * 32, 0, stream>>>(a, table);
+    sets_setup_kernel<<<1, kMaxSets + 32, 0, stream>>>(a, table);
     cudaError_t e = cudaGetLastError();
     for (int first = 0; first < sets && e == cudaSuccess; first += kDirsPerLaunch) {
         DirsArg d;

@@ -66,38 +66,34 @@ inline RowsArg single_row(const double* row)
     return a;
 }
 
-// Multi-set K2+Kf (several parameter sets in one launch): a CTA holds `per_cta` set slots of
-// `lanes` lanes each; slot q of group g is set slot_set[g * per_cta + q] (-1: empty), and the
-// sets are ordered by budget so that slot 0 of a group holds its largest.  CTA row
-// blockIdx.y = g * parent_tiles + (parent tile of the set's active list).
+// Multi-set K2+Kf (several parameter sets in one launch): grid x holds at most `blocks` CTAs, the
+// sets' side by side in proportion to their budgets (sets_ctas), grid y the parent tiles; a CTA
+// leaves partial sums of up to `lanes` parents.
 constexpr int kMaxSets = 256;
-constexpr int kMaxSlots = kMaxSets + 8;  // groups * per_cta (per_cta <= 7)
 struct SetsLayout {
-    int per_cta = 1, lanes = 64, parent_tiles = 1, groups = 1, threads = 64, blocks = 1;
+    int parent_tiles = 1, lanes = 1, blocks = 1;
 };
 SetsLayout sets_layout(int points, int sets, int waves);
-inline size_t sets_partial_doubles(const SetsLayout& L)
-{
-    return (size_t)L.groups * L.parent_tiles * L.blocks * L.threads * 3;
-}
+// First CTA of every set, and their number (first[sets]).
+void sets_ctas(const SetsLayout& L, bool fp64, int points, const int64_t* samples, int sets, uint16_t* first);
+inline size_t sets_partial_doubles(const SetsLayout& L) { return (size_t)L.parent_tiles * L.blocks * L.lanes * 3; }
 // Per-call set table in the workspace, written by launch_sets_setup.
 constexpr int kSetDirsWords = 4 * 30 + 4;  // state[4][30], shift[4]: the K2+Kf box's four dimensions
 struct SetTable {
     double* rows[kMaxSets];      // each set's table (row 0 = the initial row)
     uint32_t samples[kMaxSets];  // Sobol budget per set
-    int32_t slot_set[kMaxSlots]; // set of each slot, -1 empty
-    int32_t set_slot[kMaxSets];  // slot of each set
+    int32_t cta_first[kMaxSets + 1];  // the set's first CTA of the K2+Kf launch
     double inv[kMaxSets];        // 1 / samples (0 without NLO kernels)
     uint32_t dirs[kMaxSets][kSetDirsWords];  // Sobol directions of dimensions 0..3 and their shifts
 };
-cudaError_t launch_sets_setup(double* const* rows, const int64_t* samples, const int32_t* slot_set,
-                              const SobolDirsArg* const* dirs, int sets, int slots, bool nlo, SetTable* table,
+cudaError_t launch_sets_setup(double* const* rows, const int64_t* samples, const uint16_t* cta_first,
+                              const SobolDirsArg* const* dirs, int sets, bool nlo, SetTable* table,
                               cudaStream_t stream);
-// Sets with their own Sobol points (the set table's directions).
+// Sets with their own Sobol points (the set table's directions); blocks = cta_first[sets].
 cudaError_t launch_k2kf_sets(const nlo_bk_params& p, const double* r, int points, int sets, const double* spline,
-                             size_t spline_stride, const int32_t* active, const int32_t* counts,
-                             const nlo_bk_box& box, const SetsLayout& L, const SetTable* table, double* out,
-                             double* partial, cudaStream_t stream, bool cleared = false);
+                             const int32_t* active, const int32_t* counts, const nlo_bk_box& box, int blocks,
+                             const SetTable* table, double* out, double* partial, cudaStream_t stream,
+                             bool cleared = false);
 
 // Records a message for nlo_last_error() and returns code.
 int set_last_error(int code, const char* message);

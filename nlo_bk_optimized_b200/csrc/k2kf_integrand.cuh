@@ -495,6 +495,32 @@ __device__ __forceinline__ void k2_prepare_pair(const FastSpline& s, float cpt_s
     put(9, zsq, z2sq);
 }
 
+// Parents of a CTA of the fixed-point kernels; larger grids take several parent tiles.
+constexpr int kLaneCap = 448;
+
+// The box at the kernels' precision with the integral's constant factor.
+template <typename T>
+inline K2Box<T> make_box(const nlo_bk_params& p, const nlo_bk_box& box, bool sym)
+{
+    K2Box<T> kb;
+    double volume = 1.0;
+    for (int d = 0; d < 4; ++d) {
+        kb.lower[d] = (T)box.lower[d];
+        kb.width[d] = (T)box.width[d];
+    }
+    if (sizeof(T) == sizeof(float)) {
+        const float v01 = (float)box.width[0] * (float)box.width[1];
+        const float v23 = (float)box.width[2] * (float)box.width[3];
+        volume = (double)(v01 * v23);
+    } else {
+        volume = box.width[0] * box.width[1] * box.width[2] * box.width[3];
+    }
+    // the FP32 path folds the symmetrisation's 1/2 into the per-sample weight
+    const double half = (sizeof(T) == sizeof(float) && sym) ? 0.5 : 1.0;
+    kb.cpt_scale = (T)(half * volume * p.nc * p.nc / (8.0 * kPi * kPi * kPi * kPi));
+    return kb;
+}
+
 // The kernel instantiation of a parameter set: FP64 (one form for every coupling) or the
 // FP32 coupling variant; f(T(), SYM, COUPLING) with std::integral_constant tags.
 template <class F>
