@@ -297,7 +297,8 @@ typedef struct nlo_bk_vegas_options {
  * starts from the uniform grid with the full warm-up). */
 size_t nlo_bk_vegas_state_doubles(int32_t points, int32_t bins);
 
-/* Workspace bytes of nlo_bk_rhs_vegas / nlo_bk_evolve_vegas (at least nlo_bk_rhs_workspace_bytes). */
+/* Workspace bytes of nlo_bk_rhs_vegas / nlo_bk_evolve_vegas with these options: they depend on the
+ * samples and replicas (at least nlo_bk_rhs_workspace_bytes). */
 size_t nlo_bk_vegas_workspace_bytes(int32_t points, const nlo_bk_vegas_options* options);
 
 /* The right-hand side of nlo_bk_rhs_history with K2+Kf by Vegas for the active parents

@@ -232,8 +232,11 @@ cudaError_t launch_typed(const nlo_bk_params& p, const double* r, int points, co
     cudaGetDevice(&device);
     cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
     if (per_sm < 1) per_sm = 1;
-    uint64_t blocks = (uint64_t)per_sm * sms / (uint64_t)parent_tiles;
-    if (blocks < 1) blocks = 1;
+    // A GPU's worth of CTAs for every parent tile, not for all of them together: the tiles are
+    // filled in order, so at 449 to about 490 points the second is empty (the saturated parents are
+    // not active) and its CTAs return at once, and beyond that it has few parents.  One RK4 step,
+    // 2^18 samples: 450 points 5.1 -> 3.6 ms, 520 points 5.6 -> 4.5, 700 points 7.2 -> 6.8.
+    uint64_t blocks = (uint64_t)per_sm * sms;
     if (blocks > (uint64_t)max_blocks) blocks = (uint64_t)max_blocks;
     // The tile (a multiple of the 32 samples of an FP32 partial sum, at most one sample per thread)
     // for which a CTA's share of the samples rounds up least, with 8 samples' worth of staging a
