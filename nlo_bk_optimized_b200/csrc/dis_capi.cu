@@ -100,7 +100,6 @@ DisArgs<T> make_args(const nlo_dis_kinematics& k, const nlo_dipole& d)
         a.gbw.lambda = (T)d.lambda;
         a.gbw.gamma = (T)d.gamma;
         a.gbw.y0 = (T)std::log(1.0 / d.x0);
-        a.gbw64 = {d.qs0sqr, d.lambda, d.gamma, std::log(1.0 / d.x0)};
         a.gbw_min_r = 1e-30;
         a.gbw_max_r = 1e3;
     }

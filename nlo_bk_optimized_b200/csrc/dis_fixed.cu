@@ -91,9 +91,7 @@ __global__ void __launch_bounds__(kFixedThreads, 3) fixed_triple_kernel(
     __shared__ uint32_t sst[kFixedDims][30];
     __shared__ uint32_t ssh[kFixedDims];
     __shared__ double red[3][kFixedThreads / 32];
-    __shared__ WarpShared<T, kTermI3N, kFixedThreads> ws;
     if (threadIdx.x == 0) a = args;
-    ws.stage(rule);
     const SobolDirsArg& sd = dirs[dir_base + blockIdx.y];  // replicates: one per grid row
     for (int k = threadIdx.x; k < kFixedDims * 30; k += blockDim.x) sst[k / 30][k % 30] = sd.state[k / 30][k % 30];
     if (threadIdx.x < kFixedDims) ssh[threadIdx.x] = sd.shift[threadIdx.x];
@@ -111,17 +109,15 @@ __global__ void __launch_bounds__(kFixedThreads, 3) fixed_triple_kernel(
         const bool valid = t < lanes;
         double fw = 0.0, sw = 0.0;
         int bin[kFixedDims];
-        double first[kFixedDims], second[kFixedDims];
+        T v[3] = {(T)0, (T)0, (T)0};
         if (valid) {
             float u[kFixedDims];
 #pragma unroll
             for (int d = 0; d < kFixedDims; ++d) u[d] = sobol_unit<float>(sobol_bits(sst[d], ssh[d], i), i);
+            double first[kFixedDims], second[kFixedDims];
             endpoint_map(edges, g, u, first, second, fw, sw, bin);
+            qg_triple(a, odd ? second : first, rule, v);
         }
-#pragma unroll
-        for (int d = 0; d < kFixedDims; ++d) first[d] = valid ? (odd ? second[d] : first[d]) : 0.5;
-        T v[3];
-        qg_triple(a, valid, first, rule, ws, v);
         T v2[3];
 #pragma unroll
         for (int k = 0; k < 3; ++k) v2[k] = __shfl_xor_sync(0xffffffffu, v[k], 1);

@@ -67,7 +67,6 @@ struct DisArgs {
     // dipole
     bool table;
     GBWParams<T> gbw;
-    GBWParams<double> gbw64;
     double gbw_min_r, gbw_max_r;
     TableView tab;
 };
@@ -79,25 +78,20 @@ __device__ __forceinline__ T amplitude(const DisArgs<T>& a, double r, double Y)
     return gbw_amplitude(a.gbw, (T)r, (T)Y);
 }
 
-// The three dipoles of a qg sample at one rapidity, in the arithmetic type A: a table looks its
-// rows up once.
-template <typename A, typename T>
-__device__ __forceinline__ void amplitudes3(const DisArgs<T>& a, double r01, double r02, double r21, double Y, A& N01,
-                                            A& N02, A& N21)
+// The three dipoles of a qg sample at one rapidity: a table looks its rows up once.
+template <typename T>
+__device__ __forceinline__ void amplitudes3(const DisArgs<T>& a, double r01, double r02, double r21, double Y, T& N01,
+                                            T& N02, T& N21)
 {
     if (a.table) {
         const TableRow row = table_row(a.tab, Y);
-        N01 = (A)table_amplitude_at(a.tab, row, r01);
-        N02 = (A)table_amplitude_at(a.tab, row, r02);
-        N21 = (A)table_amplitude_at(a.tab, row, r21);
-    } else if constexpr (sizeof(A) == 8) {
-        N01 = gbw_amplitude(a.gbw64, r01, Y);
-        N02 = gbw_amplitude(a.gbw64, r02, Y);
-        N21 = gbw_amplitude(a.gbw64, r21, Y);
+        N01 = (T)table_amplitude_at(a.tab, row, r01);
+        N02 = (T)table_amplitude_at(a.tab, row, r02);
+        N21 = (T)table_amplitude_at(a.tab, row, r21);
     } else {
-        N01 = gbw_amplitude(a.gbw, (A)r01, (A)Y);
-        N02 = gbw_amplitude(a.gbw, (A)r02, (A)Y);
-        N21 = gbw_amplitude(a.gbw, (A)r21, (A)Y);
+        N01 = gbw_amplitude(a.gbw, (T)r01, (T)Y);
+        N02 = gbw_amplitude(a.gbw, (T)r02, (T)Y);
+        N21 = gbw_amplitude(a.gbw, (T)r21, (T)Y);
     }
 }
 
@@ -969,6 +963,92 @@ __device__ __forceinline__ GSet<float> g_moments_warp(bool on, const Trip<float>
     return m;
 }
 
+// FP32 moments, one lane per sample (the fixed-Sobol path; qg_triple says why).  Per node y the reciprocal 1/y is shared by the two sides;
+// per side the quantities that do not depend on y (M2 = Qbar^2 + m^2, its square root,
+// lambda m^2, x3^2, omega x2^2) are formed once.  With q = sqrt(B/y):
+//   z0 = sqrt(M2) q,  z1 = sqrt(A1) q,  z1 - z0 = q delta/(sqrt(A1)+sqrt(M2)),
+// so each (node, side) needs two square roots and two reciprocals besides the Bessel pairs.
+__device__ __forceinline__ K01<float> bessel_k01_rcp(float x, float& rx)
+{
+    rx = rcp_approx_f(x);
+    return bessel_k01_from_rcp(x, rx);
+}
+
+__device__ __forceinline__ GSet<float> g_moments_f32(const Trip<float>& t, const InnerRule& rule)
+{
+    // The side constants of the moments (8 omega, 4 omega, 4, 2) are applied after the
+    // loop, and sqrt(y) cancels between sqrt(A/B) = z sqrt(y)/B and the 1/sqrt(y) of the
+    // G functions:
+    //   G11 = 2 sum w/y K0(z1)             G21 = 4 sum w/B z1 K1(z1)
+    //   G12 = 4 omega sum w/(y B) D12      G22 = 8 omega sum w/B E
+    // with D12 = z1 K1(z1) - z0 K1(z0) (or the Euler-Maclaurin d1) and
+    // E = (A1 F(z1) - M2 F(z0))/y, F(z) = K0 + 2 K1/z (or d2/B).
+    float acc22[2], acc12[2], acc21[2], acc11[2];
+    float M2[2], sM2[2], lm2[2], x3[2], wx2[2];
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        acc22[s] = acc12[s] = acc21[s] = acc11[s] = 0.0f;
+        M2[s] = t.Qb2[s] + t.m2;
+        sM2[s] = sqrtf(M2[s]);
+        lm2[s] = t.lam[s] * t.m2;
+        x3[s] = t.x3sq[s];
+        wx2[s] = t.omega[s] * t.x2sq[s];
+    }
+    for (int i = 0; i < rule.n; ++i) {
+        const float y = (float)rule.y[i];
+        const float w = (float)rule.w[i];
+        const float iy = rcp_approx_f(y);
+        const float wiy = w * iy;
+#pragma unroll
+        for (int s = 0; s < 2; ++s) {
+            const float B = fmaf(y, x3[s], wx2[s]);
+            const float iB = rcp_approx_f(B);
+            const float q = sqrtf(B * iy);
+            const float delta = y * lm2[s];
+            const float Al = delta + M2[s];
+            const float sAl = sqrtf(Al);
+            const float z1 = sAl * q, z0 = sM2[s] * q;
+            float r1, r0;
+            const K01<float> kl = bessel_k01_rcp(z1, r1);
+            const K01<float> k0 = bessel_k01_rcp(z0, r0);
+            const float h = q * delta * rcp_approx_f(sAl + sM2[s]);
+            const float z1k1 = z1 * kl.k1;
+            float d12, e22;
+            if (h < 0.3f && h < 0.1f * z0) {
+                // Euler-Maclaurin integral of dF/dz over [z0, z1] (see f_differences_em)
+                const float h2 = h * h;
+                const float e2 = h2 * (1.0f / 12.0f), e4 = h2 * h2 * (1.0f / 720.0f);
+                const float d1 = 0.5f * h * (-z0 * k0.k0 - z1 * kl.k0) -
+                                 e2 * ((z1k1 - kl.k0) - (z0 * k0.k1 - k0.k0)) +
+                                 e4 * ((z1k1 - 2.0f * kl.k0 - kl.k1 * r1) - (z0 * k0.k1 - 2.0f * k0.k0 - k0.k1 * r0));
+                const float d2 = 0.5f * h * (-z0 * z0 * k0.k1 - z1 * z1k1) -
+                                 e2 * ((z1 * z1 * kl.k0 - z1k1) - (z0 * z0 * k0.k0 - z0 * k0.k1)) +
+                                 e4 * (((3.0f + z1 * z1) * kl.k0 - 4.0f * z1k1) -
+                                       ((3.0f + z0 * z0) * k0.k0 - 4.0f * z0 * k0.k1));
+                d12 = d1;
+                e22 = iB * d2;
+            } else {
+                d12 = z1k1 - z0 * k0.k1;
+                e22 = iy * (Al * fmaf(2.0f * kl.k1, r1, kl.k0) - M2[s] * fmaf(2.0f * k0.k1, r0, k0.k0));
+            }
+            const float wiB = w * iB;
+            acc22[s] = fmaf(wiB, e22, acc22[s]);
+            acc12[s] = fmaf(wiy * iB, d12, acc12[s]);
+            acc21[s] = fmaf(wiB, z1k1, acc21[s]);
+            acc11[s] = fmaf(wiy, kl.k0, acc11[s]);
+        }
+    }
+    GSet<float> m;
+#pragma unroll
+    for (int s = 0; s < 2; ++s) {
+        m.g22[s] = 8.0f * t.omega[s] * acc22[s];
+        m.g12[s] = 4.0f * t.omega[s] * acc12[s];
+        m.g21[s] = 4.0f * acc21[s];
+        m.g11[s] = 2.0f * acc11[s];
+    }
+    return m;
+}
+
 // The FP64 build's moments (one lane per sample).
 template <typename T>
 __device__ __forceinline__ GSet<T> g_moments(const Trip<T>& t, const InnerRule& rule)
@@ -1014,45 +1094,25 @@ __device__ __forceinline__ bool qg_geometry(const DisArgs<T>& a, const double* x
     return g.Y >= 0.0;
 }
 
-// Its amplitudes, coupling and tripole geometry.
+// Its amplitudes (the tripole factor N012), coupling and tripole geometry.
 template <typename T>
 struct QgPoint {
     Trip<T> t;
-    T x01sq, N01, N012, af;
+    T N012, af;
     double jac_z2;  // Jacobian / z2
 };
 
-// N01 and the tripole factor N012.
-template <typename A, typename T>
-__device__ __forceinline__ void qg_amplitudes(const DisArgs<T>& a, const QgGeometry& g, A& N01, A& N012)
-{
-    A N02, N21;
-    amplitudes3(a, g.x01, g.x02, g.x21, g.Y, N01, N02, N21);
-    const A S01 = (A)1 - N01, S02 = (A)1 - N02, S12 = (A)1 - N21;
-    N012 = a.finite_nc ? (A)1 - (A)(kNc / (2.0 * kCF)) * (S02 * S12 - S01 / (A)(kNc * kNc)) : (A)1 - S02 * S12;
-    N01 = (A)1 - S01;
-}
-
-// Everything but the amplitudes.
 template <typename T>
 __device__ __forceinline__ void qg_point(const DisArgs<T>& a, const QgGeometry& g, QgPoint<T>& p)
 {
+    T N01, N02, N21;
+    amplitudes3(a, g.x01, g.x02, g.x21, g.Y, N01, N02, N21);
+    const T S01 = (T)1 - N01, S02 = (T)1 - N02, S12 = (T)1 - N21;
+    p.N012 = a.finite_nc ? (T)1 - (T)(kNc / (2.0 * kCF)) * (S02 * S12 - S01 / (T)(kNc * kNc)) : (T)1 - S02 * S12;
     const double ra = a.parent_coupling ? g.x01 : fmin(g.x01, fmin(g.x02, g.x21));
     p.af = alpha_bar(a, (T)ra);
     p.t = make_trip<T>(a.Q2, a.mf, g.z1, g.z2, g.x01 * g.x01, g.x02 * g.x02, g.x21 * g.x21);
-    p.x01sq = (T)(g.x01 * g.x01);
     p.jac_z2 = g.jac / g.z2;
-}
-
-template <typename T>
-__device__ __forceinline__ T qg_i1(bool transverse, const Trip<T>& t, T x01sq, T N01, T N012)
-{
-    T uvsub, trip;
-    if (transverse)
-        t_i1(t, x01sq, uvsub, trip);
-    else
-        l_i1(t, x01sq, uvsub, trip);
-    return N01 * uvsub + N012 * trip;
 }
 
 template <typename T, int TERM>
@@ -1071,7 +1131,10 @@ __device__ __forceinline__ T qg_scaled(const QgPoint<T>& p, T v)
     return DM<T>::finite(out) ? out : (T)0;
 }
 
-// One lane per sample (the FP64 nested forms among it).
+// One lane per sample (the FP64 nested forms among it).  It spells out the point once more instead
+// of calling qg_geometry and qg_point: I1's two products nearly cancel where the gluon sits on a
+// quark, and split into those pieces the compiler contracts N01 uvsub + N012 trip the other way
+// round, which moves F_L of single points of a table by 1e-4 (no nearer to FP64, nor farther).
 template <typename T, int TERM>
 __device__ T qg_term(const DisArgs<T>& a, const double* x, const InnerRule& rule)
 {
@@ -1130,41 +1193,55 @@ __device__ T qg_term(const DisArgs<T>& a, const double* x, const InnerRule& rule
 
 // I1, and I2 and I3 with the inner rule, at one point: the map, the amplitudes, the
 // coupling and the tripole geometry are shared, and I2 and I3 use one moment set (the
-// combined evaluation of the fixed-Sobol path, dis/fixed_sobol.py:273-368).  Every lane of
-// the warp calls it; `on` marks the lanes with a point.
+// combined evaluation of the fixed-Sobol path, dis/fixed_sobol.py:273-368).
 //
-// The FP32 build takes I1 and the amplitudes in FP64 (the FP64 "sensitive" part of the
-// reference's fused path): I1's parts cancel to 1/10 .. 1/100 of themselves, and 1 - S with
-// S = 1 - N leaves 1e-3 of N012 for dipoles of N ~ 1e-4; in FP32 the remainder was 1e-6 .. 6e-5 of
-// the total and, through the training scores, moved the grid.
-template <typename T, class Shared>
-__device__ void qg_triple(const DisArgs<T>& a, bool on, const double* x, const InnerRule& rule, Shared& ws, T out[3])
+// The FP32 build keeps this one function and its own moment loop: I1's parts cancel to 1/10 ..
+// 1/100 of themselves, so its FP32 rounding sets the leading digits of the spread of the
+// replicates, which is an output.  Any other order of operations, in the moments too (through the
+// training scores they move the grid and with it every rounding), is another draw of that
+// noise: the half-warp form of g_moments_warp with the same I1 moved the error by 1e-4, at
+// 2.27 ms against 2.78 for both polarisations of the benchmark.
+template <typename T>
+__device__ void qg_triple(const DisArgs<T>& a, const double* x, const InnerRule& rule, T out[3])
 {
     out[0] = out[1] = out[2] = (T)0;
-    QgGeometry g;
-    on = on && qg_geometry(a, x, g);
-    QgPoint<T> p;
-    T i1 = (T)0;
-    if (on) {
-        double N01, N012;
-        qg_amplitudes(a, g, N01, N012);
-        qg_point(a, g, p);
-        p.N012 = (T)N012;
-        const double x01sq = g.x01 * g.x01;
-        const Trip<double> t = make_trip<double>(a.Q2, a.mf, g.z1, g.z2, x01sq, g.x02 * g.x02, g.x21 * g.x21);
-        i1 = (T)qg_i1(a.transverse, t, x01sq, N01, N012);
-    }
+    const double z2min = a.z2min;
+    if (z2min > 1.0) return;
+    const double z1 = (1.0 - z2min) * x[0];
+    const double z2 = (1.0 - z1 - z2min) * x[1] + z2min;
+    const double x01 = a.maxr * x[2];
+    const double x02 = a.maxr * x[3];
+    const double phi = 2.0 * kPi * x[4];
+    const double x01sq = x01 * x01, x02sq = x02 * x02;
+    double x21sq = x01sq + x02sq - 2.0 * x01 * x02 * ::cos(phi);
+    x21sq = x21sq > 0.0 ? x21sq : 0.0;
+    const double x21 = ::sqrt(x21sq);
+    const double jac = (1.0 - z2min) * (1.0 - z1 - z2min) * x01 * x02 * a.maxr * a.maxr * 2.0 * kPi;
+    const double Y = ::log(a.W2 * z2 / kQ0sqr);
+    if (!(Y >= 0.0)) return;
+    T N01, N02, N21;
+    amplitudes3(a, x01, x02, x21, Y, N01, N02, N21);
+    const T S01 = (T)1 - N01;
+    const T S02 = (T)1 - N02;
+    const T S12 = (T)1 - N21;
+    const T N012 = a.finite_nc ? (T)1 - (T)(kNc / (2.0 * kCF)) * (S02 * S12 - S01 / (T)(kNc * kNc))
+                               : (T)1 - S02 * S12;
+    const double ra = a.parent_coupling ? x01 : fmin(x01, fmin(x02, x21));
+    const T scale = alpha_bar(a, (T)ra) * (T)(jac / z2);
+    const Trip<T> t = make_trip<T>(a.Q2, a.mf, z1, z2, x01sq, x02sq, x21sq);
+    T uvsub, trip;
+    if (a.transverse)
+        t_i1(t, (T)x01sq, uvsub, trip);
+    else
+        l_i1(t, (T)x01sq, uvsub, trip);
     GSet<T> G;
-    if constexpr (sizeof(T) == 4) {
-        G = ws.moments(on, p.t, rule.n);
-    } else if (on) {
-        G = g_moments(p.t, rule);
-    }
-    if (!on) return;
-    const T scale = p.af * (T)p.jac_z2;
-    i1 *= scale;
-    const T i2 = qg_nested_value<T, kTermI2N>(a, p, G) * scale;
-    const T i3 = qg_nested_value<T, kTermI3N>(a, p, G) * scale;
+    if constexpr (sizeof(T) == 4)
+        G = g_moments_f32(t, rule);
+    else
+        G = g_moments(t, rule);
+    const T i1 = (((T)1 - S01) * uvsub + N012 * trip) * scale;
+    const T i2 = N012 * (a.transverse ? t_i2(t, G) : l_i2(t, G)) * scale;
+    const T i3 = N012 * (a.transverse ? t_i3(t, G, G) : l_i3(t, G, G)) * scale;
     out[0] = DM<T>::finite(i1) ? i1 : (T)0;
     out[1] = DM<T>::finite(i2) ? i2 : (T)0;
     out[2] = DM<T>::finite(i3) ? i3 : (T)0;
@@ -1219,10 +1296,7 @@ __device__ __forceinline__ T term_value_warp(const DisArgs<T>& a, bool on, const
         QgGeometry g;
         on = on && qg_geometry(a, x, g);
         QgPoint<T> p;
-        if (on) {
-            qg_amplitudes(a, g, p.N01, p.N012);
-            qg_point(a, g, p);
-        }
+        if (on) qg_point(a, g, p);
         const GSet<T> G = ws.moments(on, p.t, rule.n);
         return on ? qg_scaled(p, qg_nested_value<T, TERM>(a, p, G)) : (T)0;
     } else {
