@@ -349,6 +349,8 @@ def sobol_dirs(dims: int, seed: int) -> SobolDirs:
 
     engine = torch.quasirandom.SobolEngine(dims, scramble=True, seed=seed)
     dirs = SobolDirs()
+    if dims > len(dirs.state):
+        raise IndexError(f"Sobol directions are kept for at most {len(dirs.state)} dimensions, not {dims}")
     dirs.dims = dims
     state = engine.sobolstate.numpy().astype(np.uint32)
     shift = engine.shift.numpy().astype(np.uint32)
