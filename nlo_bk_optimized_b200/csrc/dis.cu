@@ -506,7 +506,10 @@ __global__ void vegas_finalize_kernel(double* __restrict__ state, int state_stri
     int32_t* c = counts + (size_t)job * D * bins;
     if (threadIdx.x < kStSlots) sc[threadIdx.x] = slots[threadIdx.x];
     __syncthreads();
-    if (sc[kStConverged] != 0.0) return;
+    // combine sets the flag of this very round: every thread has read it before
+    const bool converged = sc[kStConverged] != 0.0;
+    __syncthreads();
+    if (converged) return;
     const int keys = 2 + D * bins;
     const double* red = reduced + (size_t)job * keys;
     // the last thread's chain of divisions runs beside the re-binning
