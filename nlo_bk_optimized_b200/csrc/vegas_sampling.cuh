@@ -109,6 +109,8 @@ __device__ __forceinline__ void warp_hist_add(const SobolWarp<D>& s, uint32_t ba
         }
         if (!counted && active) atomicAdd(&count[d * bins + bin[d]], 1);
     }
+    // one phase: the next block's lanes find these additions (the dimensions' rows are disjoint)
+    __syncwarp();
 }
 
 // The counts of a warp's whole blocks (32 bins: one per lane), before the barrier.

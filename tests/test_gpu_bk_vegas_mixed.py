@@ -1,0 +1,76 @@
+"""The mixed build's Vegas rounds of K2+Kf (two packed blocks of 32 samples a pass) against the
+oracle in FP64 on the same points."""
+
+from __future__ import annotations
+
+import ctypes
+from types import SimpleNamespace
+
+import numpy as np
+import pytest
+import torch
+
+import oracle
+
+pytestmark = pytest.mark.gpu
+
+
+def _setup(points=24, **kw):
+    from nlo_bk_optimized_b200 import MV, BKConfig
+    from nlo_bk_optimized_b200.bk import evolution as ev
+
+    config = BKConfig(RPOINTS=points - 1, MINR=1e-5, MAXR=30.0, MCINTPOINTS=1024, PRECISION="mixed", **kw)
+    r = ev._r_grid(config, device="cuda", dtype=torch.float64)
+    N = MV(qs0sqr=0.2).dipole_amplitude(r)
+    rn, Nn = r.cpu().numpy(), N.cpu().numpy()
+    active = np.nonzero((np.arange(rn.size) > 0) & (Nn <= 0.99999))[0]
+    return SimpleNamespace(config=config, r=r, N=N, rn=rn, active=active, spline=oracle.loglog_spline(rn, Nn, 1),
+                           phys=oracle.physics(config), box=oracle.nlo_box(rn))
+
+
+def _device(s, *, bins, samples, warmup=0, iterations=1, epsrel=0.0, edges=None, seed=0):
+    """Values, edges, slots and workspace of one right-hand side; `edges` as kept grids of every parent."""
+    from nlo_bk_optimized_b200 import _native
+    from nlo_bk_optimized_b200.bk import evolution as ev
+
+    lib, points = _native.load(), s.r.numel()
+    options = ev.vegas_options_of(s.config)
+    options.bins, options.samples_per_iteration, options.warmup_samples = bins, samples, warmup
+    options.max_iterations, options.min_iterations, options.epsrel = iterations, iterations, epsrel
+    options.replicas = 0
+    grids = torch.zeros(int(lib.nlo_bk_vegas_state_doubles(points, bins)), dtype=torch.float64, device="cuda")
+    base = 4 * (bins + 1)
+    if edges is not None:
+        rows = grids.reshape(points, -1)
+        rows[:, :base] = torch.as_tensor(edges).reshape(1, base)
+        rows[:, base + 9] = 1.0  # the parent has a grid
+    ws = torch.empty(int(lib.nlo_bk_vegas_workspace_bytes(points, options)), dtype=torch.uint8, device="cuda")
+    dndy, k1, k2kf = (torch.empty_like(s.N) for _ in range(3))
+    lower, width = ev.nlo_box(float(s.r[0]), float(s.r[-1]))
+    _native.check(lib.nlo_bk_rhs_vegas(ev.params_of(s.config, _native.PRECISION_MIXED), s.r.data_ptr(), points, None,
+                                       s.N.data_ptr(), 1, 0, 1, ctypes.byref(options), _native.sobol_dirs(4, seed),
+                                       _native.box(lower, width), grids.data_ptr(), dndy.data_ptr(), k1.data_ptr(),
+                                       k2kf.data_ptr(), ws.data_ptr(), ws.numel(), _native.stream_handle(s.r.device)))
+    rows = grids.cpu().numpy().reshape(points, -1)
+    return k2kf.cpu().numpy(), rows[:, :base].reshape(points, 4, bins + 1), rows[:, base:], ws
+
+
+@pytest.mark.parametrize("bins,samples", [(32, 1005), (64, 1005), (96, 2035), (31, 1005), (33, 1005)])
+def test_histograms_keep_every_sample(bins, samples):
+    """A warp adds its blocks of 32 samples to the same rows one after the other, two blocks a pass (in
+    one conflict-free phase at 32, 64 and 96 bins).  Every sample's |w| goes once into each
+    dimension's histogram, so the four of a partial row have one sum: FP64 sums of at most 2,035
+    positive terms in other orders, 2,035 x 1.1e-16 of it."""
+    from nlo_bk_optimized_b200 import _native
+
+    s = _setup()
+    _, edges, slots, ws = _device(s, bins=bins, samples=samples)
+    assert np.array_equal(edges, _device(s, bins=bins, samples=samples)[1])
+    # up to 2,048 samples one CTA per parent: its partial row begins the workspace's Vegas part
+    keys, points = 4 + 4 * bins, s.r.numel()
+    start = int(_native.load().nlo_bk_rhs_workspace_bytes(points))
+    rows = ws[start : start + 8 * keys * points].view(torch.float64).cpu().numpy().reshape(points, keys)[s.active]
+    sums = rows[:, 2 : 2 + 4 * bins].reshape(-1, 4, bins).sum(2)
+    assert np.all(slots[s.active, 4] == samples) and np.all(sums > 0)
+    assert np.all(sums.max(1) - sums.min(1) <= 2.3e-13 * sums.max(1))
+    assert np.all(sums.min(1) >= np.abs(rows[:, 0]) * (1 - 2.3e-13))
