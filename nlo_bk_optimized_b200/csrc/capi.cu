@@ -384,17 +384,28 @@ cudaError_t raise_dynamic_smem(const void* func, size_t bytes)
     // The limit is a property of the kernel on the device, shared by every host thread:
     // only ever raise it, so that a launch prepared by one thread is never invalidated by
     // another thread lowering the limit for a smaller launch of the same kernel.
+    struct Limit {
+        size_t dynamic = 0;  // admitted dynamic bytes
+        bool known = false;
+    };
     static std::mutex lock;
-    static std::map<std::pair<int, const void*>, size_t> limits;
-    if (bytes <= 48 * 1024) return cudaSuccess;  // within the default limit
+    static std::map<std::pair<int, const void*>, Limit> limits;
     int device = 0;
     cudaError_t e = cudaGetDevice(&device);
     if (e != cudaSuccess) return e;
     std::lock_guard<std::mutex> guard(lock);
-    size_t& current = limits[{device, func}];
-    if (bytes <= current) return cudaSuccess;
+    Limit& limit = limits[{device, func}];
+    if (!limit.known) {
+        // the default admits 48 KB of the kernel's own and the dynamic shared memory together
+        cudaFuncAttributes attributes;
+        if ((e = cudaFuncGetAttributes(&attributes, func)) != cudaSuccess) return e;
+        constexpr size_t kDefault = 48 * 1024;
+        limit.dynamic = attributes.sharedSizeBytes < kDefault ? kDefault - attributes.sharedSizeBytes : 0;
+        limit.known = true;
+    }
+    if (bytes <= limit.dynamic) return cudaSuccess;
     e = cudaFuncSetAttribute(func, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
-    if (e == cudaSuccess) current = bytes;
+    if (e == cudaSuccess) limit.dynamic = bytes;
     return e;
 }
 

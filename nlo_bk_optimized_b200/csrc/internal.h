@@ -99,7 +99,7 @@ cudaError_t launch_k2kf_sets(const nlo_bk_params& p, const double* r, int points
 int set_last_error(int code, const char* message);
 
 // Raise (never lower) a kernel's dynamic shared-memory limit on the current device to at
-// least `bytes`; safe when several host threads launch the same kernel with different sizes.
+// least `bytes` where those and the kernel's own shared memory exceed the default; safe when several host threads launch the same kernel with different sizes.
 cudaError_t raise_dynamic_smem(const void* func, size_t bytes);
 // The BK kernels stage their tables and sample tiles in shared memory and read little through
 // L1: ask for the largest shared-memory carveout, once per kernel and device.

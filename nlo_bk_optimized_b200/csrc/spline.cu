@@ -206,10 +206,8 @@ cudaError_t launch_splines(const double* r, const RowsArg& N, int n, int sets, i
                            int compute_factor, double* out, cudaStream_t stream, const RhsStart& start)
 {
     const size_t smem = sizeof(double) * 7 * (size_t)n;
-    if (smem > 48 * 1024) {
-        cudaError_t e = raise_dynamic_smem((const void*)splines_kernel, smem);
-        if (e != cudaSuccess) return e;
-    }
+    const cudaError_t e = raise_dynamic_smem((const void*)splines_kernel, smem);
+    if (e != cudaSuccess) return e;
     splines_kernel<<<sets, 256, smem, stream>>>(r, N, n, force_positive, factor, compute_factor, out, start);
     return cudaGetLastError();
 }
