@@ -223,6 +223,13 @@ struct FastSpline {
     float u_top;    // n - 1
 };
 
+// The same rows for Vegas, whose grids gather the samples where the integrand cancels: what the
+// roundings of the position constants leave out, and the pair for a position from log X itself.
+struct FineSpline : FastSpline {
+    float u_scale_lo, u_off_lo;
+    float l_scale, l_scale_lo;  // 1 / h
+};
+
 struct P2S {
     float p2, S;
 };
@@ -246,6 +253,30 @@ __device__ __forceinline__ void fast_amplitude_pair(const FastSpline& s, f2 u, P
     const f2 uc = make_float2(fminf(fmaxf(u.x, -1.0f), s.u_top), fminf(fmaxf(u.y, -1.0f), s.u_top));
     const f2 shifted = __fadd2_rd(uc, bc2(8388609.0f));  // 2^23 + 1 + floor(uc)
     const f2 t = sub2(uc, sub2(shifted, bc2(8388609.0f)));
+    const float4 cx = s.coef[__float_as_int(shifted.x) - 0x4B000000];
+    const float4 cy = s.coef[__float_as_int(shifted.y) - 0x4B000000];
+    const float px = fmaf(t.x, fmaf(t.x, fmaf(t.x, cx.w, cx.z), cx.y), cx.x);
+    const float py = fmaf(t.y, fmaf(t.y, fmaf(t.y, cy.w, cy.z), cy.y), cy.x);
+    ax = {px, ex2_approx(px)};
+    ay = {py, ex2_approx(py)};
+}
+
+// The pair of amplitudes at L = log2(X^2) (scale u_scale) or log X (scale l_scale).  The row comes
+// from the rounded position; the fraction t = L scale + offset - row is formed anew from the
+// two-part constants: offset - row is exact, the fused product cancels against it with one
+// rounding of t, so t is good to 1e-7 where u - floor(u) carries the rounding of u and of both
+// constants (1e-5 at u ~ 100, which was the larger part of the FP32 error of Vegas K2+Kf).
+__device__ __forceinline__ void fine_amplitude_pair(const FineSpline& s, f2 L, float scale, float scale_lo, P2S& ax,
+                                                    P2S& ay)
+{
+    const float lo = -0.5f, hi = s.u_top + 0.5f;  // below the grid and above it: the edge rows
+    const f2 u = fma2(L, bc2(scale), bc2(s.u_off));
+    const f2 uc = make_float2(fminf(fmaxf(u.x, lo), hi), fminf(fmaxf(u.y, lo), hi));
+    // an L out of range (infinite for X = 0) meets a row without slopes: any finite t will do
+    const f2 Lc = make_float2(u.x > lo && u.x < hi ? L.x : 0.0f, u.y > lo && u.y < hi ? L.y : 0.0f);
+    const f2 shifted = __fadd2_rd(uc, bc2(8388609.0f));  // 2^23 + 1 + floor(uc)
+    const f2 a = sub2(bc2(s.u_off), sub2(shifted, bc2(8388609.0f)));
+    const f2 t = add2(fma2(Lc, bc2(scale), a), fma2(Lc, bc2(scale_lo), bc2(s.u_off_lo)));
     const float4 cx = s.coef[__float_as_int(shifted.x) - 0x4B000000];
     const float4 cy = s.coef[__float_as_int(shifted.y) - 0x4B000000];
     const float px = fmaf(t.x, fmaf(t.x, fmaf(t.x, cx.w, cx.z), cx.y), cx.x);
@@ -284,10 +315,13 @@ __device__ __forceinline__ f2 fast_ndiff2(const P2S& Ax, const P2S& Ay, const P2
     return make_float2(x.x > -0.5f ? near.x : far.x, x.y > -0.5f ? near.y : far.y);
 }
 
-template <bool SYM, int COUPLING>
-__device__ __forceinline__ void k2_pair_fast(const FastSpline& s, const Phys<float>& ph, const K2ParentF& P,
+// Kf and K2 + Kf of the pair, each 0 where the sum is not finite; with a FineSpline (Vegas) Kf and
+// K2, each 0 where it is not finite, for the caller to add in FP64.
+template <bool SYM, int COUPLING, class Spline>
+__device__ __forceinline__ void k2_pair_fast(const Spline& s, const Phys<float>& ph, const K2ParentF& P,
                                              const float4* __restrict__ rec4, f2& kfw, f2& total)
 {
+    constexpr bool FINE = std::is_same<Spline, FineSpline>::value;
     constexpr float LN2 = 0.69314718055994531f;
     constexpr float L2E = 1.4426950408889634f;
     // pair layout: float4 k holds fields 2k and 2k+1 of (sample x, sample y)
@@ -308,10 +342,15 @@ __device__ __forceinline__ void k2_pair_fast(const FastSpline& s, const Phys<flo
     const f2 Xsq = fma2(bc2(P.four_r), s1, mul2(rz, rz));  // s1 = z sin^2(theta/2)
     const f2 X2sq = fma2(bc2(P.four_r), s2, mul2(rz2, rz2));
     const f2 L2X = lg22(Xsq), L2X2 = lg22(X2sq);
-    const f2 uX = fma2(L2X, bc2(s.u_scale), bc2(s.u_off)), uX2 = fma2(L2X2, bc2(s.u_scale), bc2(s.u_off));
     P2S vXx, vXy, vX2x, vX2y;
-    fast_amplitude_pair(s, uX, vXx, vXy);
-    fast_amplitude_pair(s, uX2, vX2x, vX2y);
+    if constexpr (FINE) {
+        fine_amplitude_pair(s, L2X, s.u_scale, s.u_scale_lo, vXx, vXy);
+        fine_amplitude_pair(s, L2X2, s.u_scale, s.u_scale_lo, vX2x, vX2y);
+    } else {
+        const f2 uX = fma2(L2X, bc2(s.u_scale), bc2(s.u_off)), uX2 = fma2(L2X2, bc2(s.u_scale), bc2(s.u_off));
+        fast_amplitude_pair(s, uX, vXx, vXy);
+        fast_amplitude_pair(s, uX2, vX2x, vX2y);
+    }
     // kernels
     // log(a/b)/(a - b) = 2 (1 + hm1)/(a + b), hm1 = atanh(t)/t - 1, t = (a - b)/(a + b): the series
     // in t^2 where |a - b| < (a + b)/2, else log(a/b) directly; each case needs one reciprocal,
@@ -388,6 +427,11 @@ __device__ __forceinline__ void k2_pair_fast(const FastSpline& s, const Phys<flo
     const f2 scale = mul2(mul2(alpha, alpha), cpt);
     const f2 k2w = mul2(k2part, scale);
     kfw = mul2(make_float2(-fermion.x, -fermion.y), scale);
+    if constexpr (FINE) {
+        kfw = sel2(fabsf(kfw.x) < INFINITY, fabsf(kfw.y) < INFINITY, kfw, bc2(0.0f));
+        total = sel2(fabsf(k2w.x) < INFINITY, fabsf(k2w.y) < INFINITY, k2w, bc2(0.0f));
+        return;
+    }
     const f2 tot = add2(k2w, kfw);
     // X^2 or X'^2 below the normal range (the oracle's validity cut) gives infinite kernels
     // (the approximate reciprocal flushes denormals), so the finite test covers it
@@ -423,11 +467,23 @@ __device__ __forceinline__ FastSpline fast_spline(const float4* rows, int n, dou
     return fs;
 }
 
-__device__ __forceinline__ K2ParentF fast_parent(double r, const Phys<float>& ph)
+__device__ __forceinline__ FineSpline fine_spline(const float4* rows, int n, double x0, double h)
+{
+    FineSpline fs;
+    static_cast<FastSpline&>(fs) = fast_spline(rows, n, x0, h);
+    fs.u_scale_lo = (float)(0.5 * 0.69314718055994531 / h - (double)fs.u_scale);
+    fs.u_off_lo = (float)(-x0 / h - (double)fs.u_off);
+    fs.l_scale = (float)(1.0 / h);
+    fs.l_scale_lo = (float)(1.0 / h - (double)fs.l_scale);
+    return fs;
+}
+
+// A parent for Vegas: r^2 is that of the rounded r, as in X^2.
+__device__ __forceinline__ K2ParentF fine_parent(double r, const Phys<float>& ph)
 {
     K2ParentF P;
     P.r = (float)r;
-    P.r2 = (float)(r * r);
+    P.r2 = P.r * P.r;
     P.lr = (float)log(r);
     P.two_r = (float)(2.0 * r);
     P.four_r = (float)(4.0 * r);
@@ -437,32 +493,27 @@ __device__ __forceinline__ K2ParentF fast_parent(double r, const Phys<float>& ph
 
 // The records of two samples (component x, y) at box coordinates lz = log z, lz2 = log z',
 // th, th2, in registers, for a caller that evaluates each record once (Vegas, one parent per
-// integral): k2_prepare_x with the amplitudes from the FastSpline rows, cos th from the half
-// angle's sine and cosine, and z^2 z'^2 for the Jacobian.
-__device__ __forceinline__ void k2_prepare_pair(const FastSpline& s, float cpt_scale, f2 lz, f2 lz2, f2 th, f2 th2,
+// integral): k2_prepare_x with the amplitudes from the FineSpline rows, z^2 z'^2 for the Jacobian,
+// and every cosine as 1 - 2 sin^2 of the half angle with the 1s cancelled by hand, z' - z c12 =
+// (z' - z) + 2 z sin^2, so that neighbouring z and z' at small angles, where adapted grids put
+// their samples, keep their differences.
+__device__ __forceinline__ void k2_prepare_pair(const FineSpline& s, float cpt_scale, f2 lz, f2 lz2, f2 th, f2 th2,
                                                 float4 (&rec4)[kRecLen / 2])
 {
     constexpr float LN2 = 0.69314718055994531f;
-    constexpr float L2E = 1.4426950408889634f;
     const f2 z = make_float2(expf(lz.x), expf(lz.y)), z2 = make_float2(expf(lz2.x), expf(lz2.y));
-    f2 sh1, ch1, sh2, ch2, sh12;
-    sincosf(0.5f * th.x, &sh1.x, &ch1.x);
-    sincosf(0.5f * th.y, &sh1.y, &ch1.y);
-    sincosf(0.5f * th2.x, &sh2.x, &ch2.x);
-    sincosf(0.5f * th2.y, &sh2.y, &ch2.y);
-    sh12 = make_float2(sinf(0.5f * (th.x - th2.x)), sinf(0.5f * (th.y - th2.y)));
-    const f2 c1 = mul2(sub2(ch1, sh1), add2(ch1, sh1)), c2 = mul2(sub2(ch2, sh2), add2(ch2, sh2));
-    const f2 ss12 = mul2(sh12, sh12);
-    const f2 c12 = fma2(bc2(-2.0f), ss12, bc2(1.0f));
+    const f2 sh1 = make_float2(sinf(0.5f * th.x), sinf(0.5f * th.y));
+    const f2 sh2 = make_float2(sinf(0.5f * th2.x), sinf(0.5f * th2.y));
+    const f2 sh12 = make_float2(sinf(0.5f * (th.x - th2.x)), sinf(0.5f * (th.y - th2.y)));
+    const f2 sq1 = mul2(sh1, sh1), sq2 = mul2(sh2, sh2), sq12 = mul2(sh12, sh12);
     const f2 dz = sub2(z, z2);
     const f2 zz2 = mul2(z, z2);
-    const f2 zzsq = fma2(mul2(bc2(4.0f), zz2), ss12, mul2(dz, dz));
-    const f2 L2ZZ = lg22(zzsq);
+    const f2 zzsq = fma2(mul2(bc2(4.0f), zz2), sq12, mul2(dz, dz));
+    const f2 L2ZZ = make_float2(log2f(zzsq.x), log2f(zzsq.y));
     P2S Yx, Yy, Wx, Wy, Zx, Zy;
-    const f2 su = bc2(2.0f * L2E * s.u_scale), uo = bc2(s.u_off);
-    fast_amplitude_pair(s, fma2(lz, su, uo), Yx, Yy);
-    fast_amplitude_pair(s, fma2(lz2, su, uo), Wx, Wy);
-    fast_amplitude_pair(s, fma2(L2ZZ, bc2(s.u_scale), uo), Zx, Zy);
+    fine_amplitude_pair(s, lz, s.l_scale, s.l_scale_lo, Yx, Yy);
+    fine_amplitude_pair(s, lz2, s.l_scale, s.l_scale_lo, Wx, Wy);
+    fine_amplitude_pair(s, L2ZZ, s.u_scale, s.u_scale_lo, Zx, Zy);
     const f2 NZ = expm1_2(make_float2(LN2 * Zx.p2, LN2 * Zy.p2));  // -N_zz
     const f2 SY = make_float2(Yx.S, Yy.S), SW = make_float2(Wx.S, Wy.S), SZ = make_float2(Zx.S, Zy.S);
     const f2 dN = fast_ndiff2(Wx, Wy, Yx, Yy);  // N_Y2 - N_Y
@@ -474,11 +525,12 @@ __device__ __forceinline__ void k2_prepare_pair(const FastSpline& s, float cpt_s
     const f2 zsq = mul2(z, z), z2sq = mul2(z2, z2);
     f2 cpt = mul2(bc2(cpt_scale), mul2(zsq, z2sq));
     cpt = make_float2(ok_x ? cpt.x : 0.0f, ok_y ? cpt.y : 0.0f);
-    const f2 zc = sub2(mul2(z, c2), mul2(z2, c1));  // z cos th' - z' cos th
-    const f2 s1 = mul2(z, mul2(sh1, sh1)), s2 = mul2(z2, mul2(sh2, sh2));
+    const f2 zc = fma2(bc2(2.0f), sub2(mul2(z2, sq1), mul2(z, sq2)), dz);  // z cos th' - z' cos th
+    const f2 s1 = mul2(z, sq1), s2 = mul2(z2, sq2);
     const f2 P1 = mul2(sub2(z2, z), add2(z2, z)), P2 = mul2(mul2(bc2(-2.0f), zz2), zc);
-    const f2 U1 = sub2(z2, mul2(z, c12)), V1 = mul2(z, zc);
-    const f2 U2 = sub2(z, mul2(z2, c12)), V2 = mul2(make_float2(-z2.x, -z2.y), zc);
+    const f2 two12 = add2(sq12, sq12);
+    const f2 U1 = fma2(z, two12, make_float2(-dz.x, -dz.y)), V1 = mul2(z, zc);
+    const f2 U2 = fma2(z2, two12, dz), V2 = mul2(make_float2(-z2.x, -z2.y), zc);
     const f2 lm = make_float2(fminf(fminf(lz.x, lz2.x), 0.5f * LN2 * L2ZZ.x),
                               fminf(fminf(lz.y, lz2.y), 0.5f * LN2 * L2ZZ.y));
     const f2 Dl = mul2(bc2(2.0f), sub2(lz2, lz));

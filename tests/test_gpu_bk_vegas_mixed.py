@@ -15,13 +15,13 @@ import oracle
 pytestmark = pytest.mark.gpu
 
 
-def _setup(points=24, **kw):
+def _setup(points=24, minr=1e-5, maxr=30.0, qs0sqr=0.2, **kw):
     from nlo_bk_optimized_b200 import MV, BKConfig
     from nlo_bk_optimized_b200.bk import evolution as ev
 
-    config = BKConfig(RPOINTS=points - 1, MINR=1e-5, MAXR=30.0, MCINTPOINTS=1024, PRECISION="mixed", **kw)
+    config = BKConfig(RPOINTS=points - 1, MINR=minr, MAXR=maxr, MCINTPOINTS=1024, PRECISION="mixed", **kw)
     r = ev._r_grid(config, device="cuda", dtype=torch.float64)
-    N = MV(qs0sqr=0.2).dipole_amplitude(r)
+    N = MV(qs0sqr=qs0sqr).dipole_amplitude(r)
     rn, Nn = r.cpu().numpy(), N.cpu().numpy()
     active = np.nonzero((np.arange(rn.size) > 0) & (Nn <= 0.99999))[0]
     return SimpleNamespace(config=config, r=r, N=N, rn=rn, active=active, spline=oracle.loglog_spline(rn, Nn, 1),
@@ -29,7 +29,7 @@ def _setup(points=24, **kw):
 
 
 def _device(s, *, bins, samples, warmup=0, iterations=1, epsrel=0.0, edges=None, seed=0):
-    """Values, edges, slots and workspace of one right-hand side; `edges` as kept grids of every parent."""
+    """Values, edges, slots and workspace of one right-hand side; `edges` [points, 4 (bins + 1)]: kept grids."""
     from nlo_bk_optimized_b200 import _native
     from nlo_bk_optimized_b200.bk import evolution as ev
 
@@ -42,7 +42,7 @@ def _device(s, *, bins, samples, warmup=0, iterations=1, epsrel=0.0, edges=None,
     base = 4 * (bins + 1)
     if edges is not None:
         rows = grids.reshape(points, -1)
-        rows[:, :base] = torch.as_tensor(edges).reshape(1, base)
+        rows[:, :base] = torch.as_tensor(edges)
         rows[:, base + 9] = 1.0  # the parent has a grid
     ws = torch.empty(int(lib.nlo_bk_vegas_workspace_bytes(points, options)), dtype=torch.uint8, device="cuda")
     dndy, k1, k2kf = (torch.empty_like(s.N) for _ in range(3))
@@ -74,3 +74,27 @@ def test_histograms_keep_every_sample(bins, samples):
     assert np.all(slots[s.active, 4] == samples) and np.all(sums > 0)
     assert np.all(sums.max(1) - sums.min(1) <= 2.3e-13 * sums.max(1))
     assert np.all(sums.min(1) >= np.abs(rows[:, 0]) * (1 - 2.3e-13))
+
+
+@pytest.mark.parametrize("points,maxr,qs0sqr,samples,symmetrize", [(119, 100.0, 0.948, 36068, True),
+                                                                   (88, 100.0, 0.621, 12421, True),
+                                                                   (77, 100.0, 2.585, 16178, False)])
+def test_error_on_adapted_grids(points, maxr, qs0sqr, samples, symmetrize):
+    """One iteration on grids adapted by a warm-up and two iterations in FP64 (the oracle's), whose
+    samples gather where the integrand cancels: the vector of values over the parents keeps the
+    single-precision bound of 2e-5 (the scalar evaluation with knot-relative amplitudes keeps
+    1e-5 on average; positions rounded to FP32 in units of the grid gave up to 7e-5)."""
+    s = _setup(points, minr=1e-6, maxr=maxr, qs0sqr=qs0sqr, SYMMETRIZE_Z_Z2_INTEGRATION=symmetrize)
+    edges = np.tile(np.linspace(0, 1, 33), (points, 4, 1))
+    want = np.zeros(points)
+    for i in s.active:
+        grid = oracle.VegasGrid(None)
+        run = dict(min_iterations=1, epsrel=0.0, f32_points=True, state=grid)
+        oracle.vegas_k2kf(float(s.rn[i]), s.spline, s.phys, s.box, 0, samples=samples, warmup=samples // 5,
+                          max_iterations=2, **run | {"min_iterations": 2})
+        edges[i] = grid.edges
+        want[i] = oracle.vegas_k2kf(float(s.rn[i]), s.spline, s.phys, s.box, 0, samples=samples, warmup=0,
+                                    max_iterations=1, **run).value
+    got = _device(s, bins=32, samples=samples, edges=edges.reshape(points, -1))[0]
+    error = np.linalg.norm(got[s.active] - want[s.active]) / np.linalg.norm(want[s.active])
+    assert error <= 2e-5, error
