@@ -70,9 +70,9 @@ MUFU_PER_SM_PER_CLOCK = 16
 # spline is staged into shared memory once per CTA and each CTA writes 3 doubles per
 # parent, so the bytes do not grow with the number of samples.
 K2KF_DRAM_BYTES_PER_LAUNCH = 52224
-# Launches of our kernels per RK4 step: 4 stages of spline refit with the active list, K1, K2+Kf,
-# K2+Kf finalize, assembly with the stage combination.
-LAUNCHES_PER_RK4_STEP = 4 * 5
+# Launches of our kernels per RK4 step: 4 right-hand sides x (spline refit, active
+# list, K1, K2+Kf, K2+Kf finalize, assemble) + 4 stage combinations.
+LAUNCHES_PER_RK4_STEP = 4 * 6 + 4
 SM_COUNT = 148
 FP32_LANES_PER_SM = 128
 # CPU baseline sample: complete right-hand sides spread over the evolution

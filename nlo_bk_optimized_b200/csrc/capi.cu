@@ -218,19 +218,15 @@ int run_rhs(const nlo_bk_params& p, const double* r, const double* N, int points
         history.rows = rows;
         history.on = true;
     }
+    if ((e = launch_splines(r, single_row(N), points, 1, p.force_positive, b.factor, factor_ready ? 0 : 1, b.spline,
+                            stream, b.k1, b.k2kf)) != cudaSuccess)
+        return cuda_fail(e, "splines");
     // Sobol QMC: K2+Kf takes every active parent (a shard owns a range of Sobol indices), K1
     // the active parents i with i % shards == shard.  Vegas: both take the shard's parents.
     const bool split_samples = vegas == nullptr;
-    RhsStart start;
-    start.active = b.active;
-    start.count = b.count;
-    start.shard = split_samples ? 0 : shard;
-    start.shards = split_samples ? 1 : shards;
-    start.k1 = b.k1;
-    start.k2kf = b.k2kf;
-    if ((e = launch_splines(r, single_row(N), points, 1, p.force_positive, b.factor, factor_ready ? 0 : 1, b.spline,
-                            stream, start)) != cudaSuccess)
-        return cuda_fail(e, "splines");
+    if ((e = launch_active(single_row(N), points, 1, split_samples ? 0 : shard, split_samples ? 1 : shards, b.active,
+                           b.count, stream)) != cudaSuccess)
+        return cuda_fail(e, "active");
     const int32_t* k1_active = b.active;
     const int32_t* k1_count = b.count;
     if (shards > 1 && split_samples) {
@@ -272,9 +268,8 @@ int run_rhs(const nlo_bk_params& p, const double* r, const double* N, int points
     if (vegas && order_has_nlo(p.order) && vegas->options.replicas > 0 &&
         (e = launch_k2kf_vegas_refine(p, r, N, points, b.spline, box, *vegas, b.k1, b.k2kf, stream)) != cudaSuccess)
         return cuda_fail(e, "k2kf vegas replicas");
-    // dndy NULL: the caller assembles (launch_finish_stage)
-    if (dndy && (e = launch_assemble(b.k1, b.k2kf, points, k2kf_factor(p, samples, vegas != nullptr), dndy, k2kf_out,
-                                     stream)) != cudaSuccess)
+    if ((e = launch_assemble(b.k1, b.k2kf, points, k2kf_factor(p, samples, vegas != nullptr), dndy, k2kf_out, stream)) !=
+        cudaSuccess)
         return cuda_fail(e, "assemble");
     if (k1_out) {
         if ((e = cudaMemcpyAsync(k1_out, b.k1, sizeof(double) * points, cudaMemcpyDeviceToDevice, stream)) !=
@@ -645,21 +640,18 @@ static int evolve_rows(const nlo_bk_params* params, const double* r, int32_t poi
     const bool replay = !params->kinematical_constraint && !vegas && steps > 1 && replay_pays(points);
     StepGraph graph;
     bool recorded = false;
-    const double factor = k2kf_factor(*params, (uint64_t)samples, vegas != nullptr);
     auto step_from = [&](const double* N, double* next, int it, cudaStream_t st) {
-        int latest = 0;  // the derivative that the stage's combination assembles
         auto rhs = [&](int src, int k) {
-            const int code = run_rhs(*params, r, src < 0 ? N : tmp, points, dirs_arg, (uint64_t)samples, *box, nullptr,
+            const int code = run_rhs(*params, r, src < 0 ? N : tmp, points, dirs_arg, (uint64_t)samples, *box, kk[k],
                                      nullptr, nullptr, b, factor_ready, st, 0, 1, y, table, it + 1, &side, vegas);
-            latest = k;
             factor_ready = true;
             return code;
         };
         auto comb = [&](int nk, const int* ks, const double* coef, int dst) {
             const double* kp[4];
             for (int j = 0; j < nk; ++j) kp[j] = kk[ks[j]];
-            const cudaError_t err = launch_finish_stage(b.k1, b.k2kf, factor, kk[latest], N, kp, coef, nk, points,
-                                                        dst ? next : tmp, dst ? clamp : 0, dst ? status : nullptr, st);
+            const cudaError_t err = launch_axpy_stage(N, kp, coef, nk, points, dst ? next : tmp, dst ? clamp : 0,
+                                                      dst ? status : nullptr, st);
             return err == cudaSuccess ? NLO_OK : cuda_fail(err, "stage");
         };
         return step_sequence(stepper, step, rhs, comb);
@@ -905,15 +897,12 @@ int nlo_bk_evolve_sets(const nlo_bk_params* params, const double* r, int32_t poi
         int latest = 0;  // the derivative that the stage's combination assembles
         auto rhs = [&](int src, int k) {
             const RowsArg& in = src < 0 ? now : work;
-            RhsStart start;
-            start.active = active;
-            start.count = counts;
-            start.k1 = k1;
-            start.k2kf = k2kf;
             if ((e = launch_splines(r, in, points, sets, params->force_positive, factor, factor_ready ? 0 : 1, spline,
-                                    s, start)) != cudaSuccess)
+                                    s, k1, k2kf)) != cudaSuccess)
                 return cuda_fail(e, "splines");
             factor_ready = true;
+            if ((e = launch_active(in, points, sets, 0, 1, active, counts, s)) != cudaSuccess)
+                return cuda_fail(e, "active");
             latest = k;
             const bool beside = side.ok;
             cudaStream_t k1_stream = beside ? side.aux : s;

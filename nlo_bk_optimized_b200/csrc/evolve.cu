@@ -55,20 +55,9 @@ __global__ void axpy_stage_kernel(const double* N, StageArgs a, int n, double* o
     out[i] = combined(N[i], a, i, clamp, status);
 }
 
-// The end of a stage in one launch: the derivative of each parent, then the stage combination,
-// whose terms read this thread's element only (the last of them just written).
-__global__ void finish_stage_kernel(const double* __restrict__ k1, const double* __restrict__ k2kf, double factor,
-                                    double* dndy, const double* N, StageArgs a, int n, double* out, int clamp,
-                                    uint32_t* __restrict__ status)
-{
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    double nlo;
-    dndy[i] = assembled(k1[i], k2kf + 3 * (size_t)i, factor, nlo);
-    out[i] = combined(N[i], a, i, clamp, status);
-}
-
-// Several parameter sets: blockIdx.y is the set.
+// Several parameter sets (blockIdx.y): the end of a stage in one launch, the derivative of each parent
+// and then the stage combination, whose terms read this thread's element only (the last of them
+// just written).
 __global__ void finish_stage_sets_kernel(const double* __restrict__ k1, const double* __restrict__ k2kf,
                                          const SetTable* __restrict__ table, double* dndy, RowsArg N, StageArgs a,
                                          int n, RowsArg out, int clamp, uint32_t* __restrict__ status)
@@ -166,15 +155,6 @@ static StageArgs stage_args(const double* const* k, const double* coef, int nk)
         a.c[j] = j < nk ? coef[j] : 0.0;
     }
     return a;
-}
-
-cudaError_t launch_finish_stage(const double* k1, const double* k2kf, double factor, double* dndy, const double* N,
-                                const double* const* k, const double* coef, int nk, int points, double* out,
-                                int clamp, uint32_t* status, cudaStream_t stream)
-{
-    finish_stage_kernel<<<(points + 127) / 128, 128, 0, stream>>>(k1, k2kf, factor, dndy, N, stage_args(k, coef, nk),
-                                                                  points, out, clamp, status);
-    return cudaGetLastError();
 }
 
 cudaError_t launch_finish_stage_sets(const double* k1, const double* k2kf, const SetTable* table, double* dndy,

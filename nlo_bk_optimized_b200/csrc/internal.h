@@ -105,21 +105,11 @@ cudaError_t raise_dynamic_smem(const void* func, size_t bytes);
 // L1: ask for the largest shared-memory carveout, once per kernel and device.
 cudaError_t prefer_shared_carveout(const void* func);
 
-// What a right-hand side begins with besides the refit (NULL: left out): the active parents of
-// each row (index % shards == shard; active + s * n, count + s) and the cleared K1 (+ s * n) and
-// K2+Kf sums (+ s * 3n).
-struct RhsStart {
-    int32_t* active = nullptr;
-    int32_t* count = nullptr;
-    int shard = 0, shards = 1;
-    double* k1 = nullptr;
-    double* k2kf = nullptr;
-};
 // Spline tables of `sets` rows: set s reads N.at(s) and writes out + s * spline_doubles(n)
-// and its factorisation at factor + s * 2n.
+// and its factorisation at factor + s * 2n; k1 (+ s * n) and k2kf (+ s * 3n), where given, are cleared.
 cudaError_t launch_splines(const double* r, const RowsArg& N, int n, int sets, int force_positive, double* factor,
-                           int compute_factor, double* out, cudaStream_t stream,
-                           const RhsStart& start = RhsStart());
+                           int compute_factor, double* out, cudaStream_t stream, double* k1 = nullptr,
+                           double* k2kf = nullptr);
 // active parents (index > 0, N <= 0.99999) with index % shards == shard; set s reads N.at(s)
 // and writes active + s * n and count + s
 cudaError_t launch_active(const RowsArg& N, int n, int sets, int shard, int shards, int32_t* active, int32_t* count,
@@ -182,10 +172,6 @@ cudaError_t vegas_launch_reduce(const double* partial, int keys, int blocks_per_
 
 cudaError_t launch_assemble(const double* k1, const double* k2kf, int points, double inv_samples, double* dndy,
                             double* k2kf_total, cudaStream_t stream);
-// launch_assemble into dndy, then launch_axpy_stage whose last term k[nk - 1] is dndy.
-cudaError_t launch_finish_stage(const double* k1, const double* k2kf, double factor, double* dndy, const double* N,
-                                const double* const* k, const double* coef, int nk, int points, double* out,
-                                int clamp, uint32_t* status, cudaStream_t stream);
 cudaError_t launch_axpy_stage(const double* N, const double* const* k, const double* coef, int nk, int points,
                               double* out, int clamp, uint32_t* status, cudaStream_t stream);
 // Several sets: dndy + s * points = k1 + s * points + (k2kf + s * 3 points) * table->inv[s], then

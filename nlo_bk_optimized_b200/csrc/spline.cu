@@ -50,48 +50,18 @@ __device__ __forceinline__ void warp_affine_scan(const double* a, double* c, int
     }
 }
 
-// The active parents of a row (index > 0 and N <= 0.99999, bk/evolution.py:501; index % shards ==
-// shard), compacted in index order by a ballot scan; called by all threads of a CTA.
-__device__ __forceinline__ void compact_active(const double* __restrict__ N, int n, int shard, int shards,
-                                               int32_t* __restrict__ active, int32_t* __restrict__ count)
-{
-    __shared__ int warp_counts[32];
-    __shared__ int base;
-    if (threadIdx.x == 0) base = 0;
-    __syncthreads();
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    for (int start = 0; start < n; start += blockDim.x) {
-        const int i = start + threadIdx.x;
-        const bool on = i < n && i > 0 && N[i] <= 0.99999 && i % shards == shard;
-        const unsigned mask = __ballot_sync(0xffffffffu, on);
-        if (lane == 0) warp_counts[warp] = __popc(mask);
-        __syncthreads();
-        int offset = base;
-        for (int w = 0; w < warp; ++w) offset += warp_counts[w];
-        if (on) active[offset + __popc(mask & ((1u << lane) - 1u))] = i;
-        __syncthreads();
-        if (threadIdx.x == 0) {
-            int total = 0;
-            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) total += warp_counts[w];
-            base += total;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *count = base;
-}
-
 // factor: [2][n] = 1/denominator and upper coefficient of the Thomas sweep for
 // the natural-spline system on the knots log r (it depends on the grid only).
 // With compute_factor set, one warp forms it first (and stores it for later calls).
 // One CTA per set (blockIdx.x): row N.at(set), tables at out + set * spline_doubles(n), its own
-// factorisation copy at factor + set * 2n.  `start` (optional buffers): the active list of
-// the row and the cleared sums of the right-hand side that begins with this refit, which
-// were two more launches and two more memsets on its critical path.
+// factorisation copy at factor + set * 2n.  k1 and k2kf (optional): the sums of the right-hand side
+// that begins with this refit, cleared here instead of by two memsets on its critical path.
 // What bounds it: the latency of the dependent sweeps (33 us for 400 knots with one thread per
 // row; the scans leave about 8).
 __global__ void __launch_bounds__(256) splines_kernel(const double* __restrict__ r, RowsArg rows,
                                                       int n, int force_positive, double* __restrict__ factor,
-                                                      int compute_factor, double* __restrict__ out, RhsStart start)
+                                                      int compute_factor, double* __restrict__ out,
+                                                      double* __restrict__ k1, double* __restrict__ k2kf)
 {
     const double* __restrict__ N = rows.at(blockIdx.x);
     factor += (size_t)blockIdx.x * 2 * n;
@@ -115,10 +85,10 @@ __global__ void __launch_bounds__(256) splines_kernel(const double* __restrict__
         double ns = v;
         if (force_positive && ns < 0.0) ns = 0.0;
         y[n + i] = ns < 1.0 ? log1p(-ns) : kMinLog;
-        if (start.k1) start.k1[(size_t)blockIdx.x * n + i] = 0.0;
+        if (k1) k1[(size_t)blockIdx.x * n + i] = 0.0;
     }
-    if (start.k2kf)
-        for (int i = threadIdx.x; i < 3 * n; i += blockDim.x) start.k2kf[(size_t)blockIdx.x * 3 * n + i] = 0.0;
+    if (k2kf)
+        for (int i = threadIdx.x; i < 3 * n; i += blockDim.x) k2kf[(size_t)blockIdx.x * 3 * n + i] = 0.0;
     __syncthreads();
     if (compute_factor && threadIdx.x < 32 && m >= 1) {
         // denominators of the forward sweep (interpolation.py:124-149): lane l its own stretch,
@@ -177,16 +147,39 @@ __global__ void __launch_bounds__(256) splines_kernel(const double* __restrict__
         c[2] = sl / 2.0;
         c[3] = (sr - sl) / (6.0 * h);
     }
-    if (start.active)
-        compact_active(N, n, start.shard, start.shards, start.active + (size_t)blockIdx.x * n,
-                       start.count + blockIdx.x);
 }
 
-// The active list alone, one CTA per set (blockIdx.x).
+// The active parents of each row (index > 0 and N <= 0.99999, bk/evolution.py:501; index % shards ==
+// shard), compacted in index order by a ballot scan; one CTA per set (blockIdx.x).
 __global__ void __launch_bounds__(1024) active_kernel(RowsArg rows, int n, int shard, int shards,
                                                       int32_t* __restrict__ active, int32_t* __restrict__ count)
 {
-    compact_active(rows.at(blockIdx.x), n, shard, shards, active + (size_t)blockIdx.x * n, count + blockIdx.x);
+    const double* __restrict__ N = rows.at(blockIdx.x);
+    active += (size_t)blockIdx.x * n;
+    count += blockIdx.x;
+    __shared__ int warp_counts[32];
+    __shared__ int base;
+    if (threadIdx.x == 0) base = 0;
+    __syncthreads();
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    for (int start = 0; start < n; start += blockDim.x) {
+        const int i = start + threadIdx.x;
+        const bool on = i < n && i > 0 && N[i] <= 0.99999 && i % shards == shard;
+        const unsigned mask = __ballot_sync(0xffffffffu, on);
+        if (lane == 0) warp_counts[warp] = __popc(mask);
+        __syncthreads();
+        int offset = base;
+        for (int w = 0; w < warp; ++w) offset += warp_counts[w];
+        if (on) active[offset + __popc(mask & ((1u << lane) - 1u))] = i;
+        __syncthreads();
+        if (threadIdx.x == 0) {
+            int total = 0;
+            for (int w = 0; w < (int)(blockDim.x >> 5); ++w) total += warp_counts[w];
+            base += total;
+        }
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) *count = base;
 }
 
 template <typename T>
@@ -203,12 +196,12 @@ __global__ void sobol_draw_kernel(SobolDirsArg dirs, uint64_t offset, uint64_t n
 }
 
 cudaError_t launch_splines(const double* r, const RowsArg& N, int n, int sets, int force_positive, double* factor,
-                           int compute_factor, double* out, cudaStream_t stream, const RhsStart& start)
+                           int compute_factor, double* out, cudaStream_t stream, double* k1, double* k2kf)
 {
     const size_t smem = sizeof(double) * 7 * (size_t)n;
     const cudaError_t e = raise_dynamic_smem((const void*)splines_kernel, smem);
     if (e != cudaSuccess) return e;
-    splines_kernel<<<sets, 256, smem, stream>>>(r, N, n, force_positive, factor, compute_factor, out, start);
+    splines_kernel<<<sets, 256, smem, stream>>>(r, N, n, force_positive, factor, compute_factor, out, k1, k2kf);
     return cudaGetLastError();
 }
 

@@ -4,7 +4,7 @@ launch has raised a limit before.
 
 * the nested mixed DIS terms: 27,904 B static + 420 B a bin cross at 51 bins; 118 bins cross by the
   dynamic part alone; 256 is the largest number;
-* the spline refit: 144 B + 56 B a knot, crossing at 876 knots; the dynamic part alone at 878;
+* the spline refit: 56 B a knot, crossing at 878 knots (a static part of 144 B once made it 876);
 * the BK Vegas rounds: 1,328 B + 368 B a bin + the tables, crossing at 903 knots with 32 bins in FP64
   (dynamic alone at 936) and at 129 bins with 24 knots in FP32 (133); grids long enough to cross
   at 32 bins in FP32 exceed the shared memory of K1.
