@@ -98,3 +98,40 @@ def test_error_on_adapted_grids(points, maxr, qs0sqr, samples, symmetrize):
     got = _device(s, bins=32, samples=samples, edges=edges.reshape(points, -1))[0]
     error = np.linalg.norm(got[s.active] - want[s.active]) / np.linalg.norm(want[s.active])
     assert error <= 2e-5, error
+
+
+def _couplings():
+    from nlo_bk_optimized_b200.bk.config import RunningCouplingLO as LO, RunningCouplingNLO as NLO
+
+    return {"smooth": {}, "capped": {"ALPHA_S_CAP": 0.3}, "fixed": {"RC_LO": LO.FIXED_LO, "RC_NLO": NLO.FIXED_NLO},
+            "thresholds": {"NF": 5}, "parent": {"RC_NLO": NLO.PARENT_NLO}, "gluons": {"NF": 0}}
+
+
+@pytest.mark.parametrize("symmetrize", [True, False])
+@pytest.mark.parametrize("coupling,bins,warmup,samples", [("smooth", 32, 13, 4096), ("capped", 31, 45, 2035),
+                                                          ("fixed", 33, 1005, 4099), ("thresholds", 50, 31, 5003),
+                                                          ("parent", 64, 77, 2035), ("gluons", 2, 2, 33)])
+def test_ragged_rounds_of_every_variant(symmetrize, coupling, bins, warmup, samples, monkeypatch):
+    """Every instantiation of the packed evaluation, in an iteration that starts inside a block of 32
+    points (after the warm-up) and ends in one.  The grid of the iteration is the device's own (a
+    first call whose one iteration takes the warm-up's points leaves the same one), so that the
+    oracle evaluates at the same points.  Tolerance: a sample's FP32 error is a few roundings of
+    z over its distance to the parent, 4 x 6e-8 / (X/r) of it, and among the 1e5 evaluations of a case
+    X/r reaches down to some 5e-4: 5e-4 of such a sample, which weighs no more than the value and
+    its statistical error."""
+    s = _setup(SYMMETRIZE_Z_Z2_INTEGRATION=symmetrize, **_couplings()[coupling])
+    edges = _device(s, bins=bins, samples=warmup)[1]
+    got, _, slots, _ = _device(s, bins=bins, samples=samples, warmup=warmup)
+    draw = oracle.sobol
+    monkeypatch.setattr(oracle, "sobol", lambda state, shift, offset, n, **kw: draw(state, shift, offset + warmup, n,
+                                                                                    **kw))
+    want, scale, parts = (np.zeros(s.r.numel()) for _ in range(3))
+    for i in s.active:
+        ref = oracle.vegas_k2kf(float(s.rn[i]), s.spline, s.phys, s.box, 0, samples=samples, warmup=0, bins=bins,
+                                max_iterations=1, min_iterations=1, epsrel=0.0, f32_points=True,
+                                state=oracle.VegasGrid(edges[i].copy()))
+        want[i], scale[i], parts[i] = ref.value, abs(ref.value) + ref.error, ref.components[0]
+        assert slots[i, 4] == warmup + samples
+    a = s.active
+    assert np.linalg.norm(got[a] - want[a]) <= 5e-4 * np.linalg.norm(scale[a])
+    assert np.linalg.norm(slots[a, 13] / slots[a, 1] - parts[a]) <= 5e-4 * np.linalg.norm(scale[a])
