@@ -341,10 +341,10 @@ __global__ void gauss_legendre_kernel(const DisArgs<T>* __restrict__ args, Inner
 
 // partial layout per (job, block): [total, total2, hist[D][bins]] doubles and
 // count[D][bins] int32 in a parallel array
-// CTAs per SM the register bound aims at: the FP32 LO and dipole terms are latency-bound
-// and run faster at four (64 registers); the qqbar-g terms keep three (80 registers),
-// where the nested ones issue an instruction nearly every cycle and I1 gains nothing
-// from a fourth CTA but spills.
+// CTAs per SM the register bound aims at: the FP32 LO and dipole terms are latency-bound and run
+// faster at four (64 registers), and so do the nested qqbar-g terms with their nodes on the lanes
+// (sigma_r of 24 points 24.8 ms, 25.1 at three); the other qqbar-g terms keep three (80
+// registers), where I1 gains nothing from a fourth CTA but spills.
 template <typename T, int TERM>
 constexpr int vegas_min_blocks()
 {
