@@ -944,7 +944,8 @@ __device__ __forceinline__ GSet<float> g_moments_warp(bool on, const Trip<float>
         v += __shfl_xor_sync(0xffffffffu, up4 ? u0 : u1, 4);
         v += __shfl_xor_sync(0xffffffffu, v, 2);
         v += __shfl_xor_sync(0xffffffffu, v, 1);
-        // every lane has read the segment before the shuffles: its row takes the sums
+        // its row takes the sums, once every lane has read the segment (shuffles order no memory)
+        __syncwarp();
         if (mine && (lane & 3) == 0) reinterpret_cast<float*>(side)[l >> 2] = v;
     }
     __syncwarp();

@@ -31,3 +31,19 @@ def test_points_per_warp(per_warp, extra):
     # every point has its own value, the last ones too
     tail = slice(-64, None)
     assert np.linalg.norm(got[tail] - ref[tail]) <= 1e-4 * np.linalg.norm(ref[tail])
+
+
+@pytest.mark.parametrize("inner", [8, 17, 48])
+def test_values_repeat(inner):
+    """The half-warps of a pair take their sums' place in the rows that both have read: the same bits
+    on every call, at rules that leave lanes without a node and at more points than one pass takes."""
+    from nlo_bk_optimized_b200.dipole import GBW
+    from nlo_bk_optimized_b200.dis import DISConfig, Polarization, Quark, QuarkType, integrand_qg_nested_massive
+
+    quark = Quark(QuarkType.LIGHT, 0.14)
+    config = DISConfig(quarks=(quark,), cuda_nested_points=inner)
+    x = torch.rand((90001, 5), generator=torch.Generator().manual_seed(inner)).clamp(0.02, 0.98).cuda()
+    call = lambda: integrand_qg_nested_massive(x, torch.tensor(8.0), torch.tensor(1e-3), Polarization.L, quark, "I2",  # noqa: E731
+                                               GBW(Qs0sqr=0.25, lambda_=0.29), config)
+    first = call()
+    assert all(torch.equal(first, call()) for _ in range(4))
