@@ -287,7 +287,7 @@ __global__ void __launch_bounds__(kThreads, (sizeof(T) == 4 ? 3 : 2)) round_kern
     }
 }
 
-// Per integral: add the round's partial rows in a fixed order (kSlices interleaved chains per
+// Per integral: add the round's partial rows in a fixed order (four interleaved chains per
 // key, then the chains), re-bin the grid from the histogram and, for an iteration, fold its
 // estimate into the weighted combination (value, error, convergence) and the K2 / Kf
 // components; then advance the Sobol offset.
