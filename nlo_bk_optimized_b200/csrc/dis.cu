@@ -257,8 +257,12 @@ __global__ void table_initialize_kernel(double* table, int nr, int ny, double Y)
 constexpr int kPointsThreads = 128;
 
 // A warp takes per_warp points at a time (32 but for the nested FP32 terms, see launch_points_t).
+// Eight CTAs per SM (64 registers) in FP32, four in FP64: the terms are latency-bound.  200,000 points
+// of I1, I2 and I3: 11.9, 14.4 and 17.8 us in FP32, 27.3, 42.0 and 59.0 in FP64; bounded for one CTA
+// (130 to 230 registers) 17.5, 20.6, 23.7 and 42.9, 58.2, 80.0, and FP64 at eight loses 2 us to spills
+// on few points.
 template <typename T, int TERM>
-__global__ void __launch_bounds__(kPointsThreads, (warp_term<T, TERM>() ? 8 : 1))
+__global__ void __launch_bounds__(kPointsThreads, (sizeof(T) == 4 ? 8 : 4))
     points_kernel(const DisArgs<T> args, InnerRule rule, const double* __restrict__ x, int64_t n, int per_warp,
                   double* __restrict__ out)
 {
